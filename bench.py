@@ -619,8 +619,10 @@ def run_ours(args):
         except Exception as ex:  # the GPU line is still reported
             cpu = {"error": f"{type(ex).__name__}: {ex}"}
     if rank == 0:
-        tc = {m: {"family": ["p+v kernels", "one kernel per step"][tim["kernel_family"][i]],
-                  "tile": f"64x{tim['tile_cols'][i]}",
+        tc = {m: {"family": ["p+v kernels", "one kernel per step",
+                             "on-chip time loop"][tim["kernel_family"][i]],
+                  "tile": (f"64x{tim['tile_cols'][i]}" if tim["kernel_family"][i] != 2 else
+                           f"{tim['tile_cols'][i]} columns per CTA"),
                   "ctas_per_sm": ([tim["ctas_per_sm"][i], tim["ctas_per_sm_v"][i]]
                                   if tim["kernel_family"][i] == 0 else tim["ctas_per_sm"][i]),
                   "shots_per_launch": tim["shots_per_launch"][i]}

@@ -75,8 +75,11 @@ enum daw_option {
                                 reverse order.  No counterpart in the reference, which
                                 keeps whole histories. */,
   DAW_OPT_STEP_KERNEL = 9,   /* TMA kernel family (DAW_OPT_CHUNK = 0): 0 (default) =
-                                separate pressure and velocity kernels, shots per launch
-                                and CTAs per SM chosen by the autotuner; 1 = one kernel
+                                the time loop on chip where the grid fits the SMs'
+                                registers, shared and tensor memory, else (and with
+                                DAW_OPT_PDL) separate pressure and velocity kernels,
+                                shots per launch and CTAs per SM chosen by the
+                                autotuner; 1 = one kernel
                                 per time step (pressure recomputed on the velocity
                                 stencil's halo, two alternating state sets), tile width
                                 and CTAs per SM autotuned; 2 = the family autotuned too
@@ -275,10 +278,11 @@ typedef struct daw_timing {
   int64_t kernel_launches;    /* kernels launched by the library */
   double shot_steps_fwd, shot_steps_a, shot_steps_b;  /* shot time steps by kind */
   /* TMA kernels of the last run of each mode (forward, stage A, stage B, final
-   * esource), as the autotuner chose them: family (0 = separate pressure and
-   * velocity kernels, 1 = one kernel per step), tile columns, CTAs per SM
-   * (separate kernels: of the pressure kernel) and CTAs per SM of the
-   * velocity kernel (0 for one kernel per step); zeros = not run */
+   * esource): family (0 = separate pressure and velocity kernels, 1 = one kernel
+   * per step, both with launch shapes the autotuner chose; 2 = time loop on
+   * chip), tile columns (on chip: columns per CTA), CTAs per SM (separate
+   * kernels: of the pressure kernel) and CTAs per SM of the velocity kernel
+   * (0 for the other families); zeros = not run */
   int32_t kernel_family[4], tile_cols[4], ctas_per_sm[4], ctas_per_sm_v[4];
   int32_t shots_per_launch[4]; /* shots whose time loops share one launch */
 } daw_timing;

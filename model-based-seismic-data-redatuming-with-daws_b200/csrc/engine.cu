@@ -3,12 +3,14 @@
 // driver, the mode-1 shot pipeline with on-the-fly datum extraction, and the
 // C ABI of include/daw_b200.h.
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -17,6 +19,7 @@
 #include "daw_internal.h"
 #include "fused.cuh"
 #include "kernels.cuh"
+#include "resident.cuh"
 
 using namespace daw;
 
@@ -130,6 +133,20 @@ void sponge_b(int npml, int n, std::vector<float>& d, std::vector<float>& d1) {
   }
 }
 
+// Host view of a station map, for planning the on-chip time loops: per column
+// the touched rows (lo > hi: none), the most entries of a point and the range
+// of its stations, and the bounding box of all touched points.
+struct MapInfo {
+  std::vector<int> lo, hi, cnt, smin, smax;
+  int r0 = INT_MAX, r1 = -1, c0 = INT_MAX, c1 = -1;  // inclusive; r1 < r0: empty
+};
+
+// A station map's injection tables for CTAs of C columns (resident.cuh).
+struct ResTables {
+  int C = 0;
+  ResidentInj dev{};
+};
+
 // Per-shot device context of the pipeline.
 struct ShotCtx {
   int shot = 0, nt = 0, nr = 0, nd = 0;
@@ -141,6 +158,8 @@ struct ShotCtx {
   std::string tag;
   StationsDev rec, src;
   InjMapDev recmap, srcmap;
+  MapInfo recinfo, srcinfo;
+  ResTables rectab, srctab;
   float *d_s = nullptr, *d_dobs = nullptr, *d_datar = nullptr, *d_deltadr = nullptr;
   float *d_deltade = nullptr, *d_dataesc = nullptr, *d_datae = nullptr;
   float *d_redF = nullptr, *d_redE = nullptr, *d_red = nullptr, *d_redf = nullptr;
@@ -232,6 +251,7 @@ struct daw_handle {
     float us_per_step;     // measured device time of one step per shot (0: not measured)
   };
   std::map<std::string, Tuned> tuned;
+  unsigned res_tag = 1;  // next step tag of the on-chip time loops
 };
 
 namespace {
@@ -300,7 +320,8 @@ StationsDev make_stations(daw_handle* h, Pool& pool, const std::string& name, co
 }
 
 // Gather-form injection map of stations `tab` on the extended grid.
-InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int32_t* tab, int n) {
+InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int32_t* tab, int n,
+                   MapInfo* info) {
   const Grid& g = h->g;
   struct E {
     long long pt;
@@ -385,6 +406,21 @@ InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int
       cbase[c] = idx;
       if (chi[c] >= clo[c]) idx += chi[c] - clo[c] + 1;
     }
+  }
+  info->lo = clo;
+  info->hi = chi;
+  info->cnt.assign(g.n2e, 0);
+  info->smin.assign(g.n2e, INT_MAX);
+  info->smax.assign(g.n2e, -1);
+  for (size_t q = 0; q < pt.size(); ++q) {
+    const int c = pt[q] / g.ld, r = pt[q] % g.ld;
+    info->cnt[c] = std::max(info->cnt[c], ptr[q + 1] - ptr[q]);
+    info->smin[c] = std::min(info->smin[c], sta[ptr[q]]);  // entries are in station order
+    info->smax[c] = std::max(info->smax[c], sta[ptr[q + 1] - 1]);
+    info->r0 = std::min(info->r0, r);
+    info->r1 = std::max(info->r1, r);
+    info->c0 = std::min(info->c0, c);
+    info->c1 = std::max(info->c1, c);
   }
   InjMapDev m;
   m.npts = (int)pt.size();
@@ -576,6 +612,8 @@ struct Batch {
   std::vector<ShotDevice> h_shots;
   int max_nt = 0, max_rec = 0, max_datum = 0;
   bool no_datum = false;  // forward-only batches: no datum gathers
+  bool resident = false;  // the run's time loops stay on chip (resident.cuh)
+  int res_cols = 0;       // with that many columns per CTA
   int slot0 = 0;
 };
 
@@ -855,6 +893,338 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
   return best;
 }
 
+// ---------------------------------------------------------------------------
+// Time loops on chip (stencil_resident.cu): planning and launches.
+// ---------------------------------------------------------------------------
+// Bytes of the rectangle buffers per launch (the time loop is cut into
+// launches of as many steps as fit) and the most a step may need of it: below
+// that, reloading the state at a cut (two passes over it) stays small beside
+// the steps between the cuts.
+constexpr size_t kRectBytes = (size_t)512 << 20, kRectStepBytes = (size_t)4 << 20;
+
+bool resident_family(const daw_handle* h) {
+  return tma_path(h) && h->opt.step == 0 && !h->opt.pdl;
+}
+
+// Launches that wait on one another's CTAs must not overlap another handle's
+// of the same device: each launch follows the last one of the process.
+struct ResidentOrder {
+  std::mutex mu;
+  std::map<int, std::pair<cudaEvent_t, const daw_handle*>> last;
+};
+ResidentOrder& resident_order() {
+  static ResidentOrder o;
+  return o;
+}
+
+// Per-CTA headers (first row, rows, first station, stations) of a map for C
+// columns per CTA and the table capacities; false when a source touches a row
+// or column that the stencil never updates (off points from the far edges).
+bool resident_heads(const Grid& g, const MapInfo& info, int C, int off, std::vector<int4>* heads,
+                    int* pts, int* m, int* nsta) {
+  *pts = *m = *nsta = 0;
+  const int G = (g.n2e + C - 1) / C;
+  if (heads) heads->assign(G, make_int4(0, 0, 0, 0));
+  if (info.r1 < info.r0) return true;
+  if (info.r0 < 2 || info.r1 >= g.n1e - off || info.c0 < 2 || info.c1 >= g.n2e - off) return false;
+  for (int b = 0; b < G; ++b) {
+    int lo = INT_MAX, hi = -1, s0 = INT_MAX, s1 = -1;
+    for (int c = b * C; c < std::min(g.n2e, (b + 1) * C); ++c) {
+      if (info.hi[c] < info.lo[c]) continue;
+      lo = std::min(lo, info.lo[c]);
+      hi = std::max(hi, info.hi[c]);
+      s0 = std::min(s0, info.smin[c]);
+      s1 = std::max(s1, info.smax[c]);
+      *m = std::max(*m, info.cnt[c]);
+    }
+    if (hi < lo) continue;
+    lo &= ~1;
+    const int rows = (hi | 1) - lo + 1;
+    if (heads) (*heads)[b] = make_int4(lo, rows, s0, s1 - s0 + 1);
+    *pts = std::max(*pts, C * rows);
+    *nsta = std::max(*nsta, s1 - s0 + 1);
+  }
+  *m = (*m + 1) & ~1;
+  return true;
+}
+
+// Rectangles (rows, columns; end exclusive) whose pressure the gathers of a
+// run of `mode` need: the receivers' and the datum's.
+struct Box {
+  int r0 = 0, r1 = 0, c0 = 0, c1 = 0;
+  size_t elems() const { return r1 > r0 ? (size_t)(r1 - r0) * (c1 - c0) : 0; }
+};
+void gather_boxes(const daw_handle* h, const Batch& b, const ShotCtx& c, int mode, Box out[2]) {
+  const Grid& g = h->g;
+  if (mode == FM_STAGE_A || c.type_rec != 0) return;
+  const MapInfo& i = c.recinfo;
+  if (i.r1 >= i.r0) out[0] = Box{i.r0, i.r1 + 1, i.c0, i.c1 + 1};
+  if (h->ndatum > 0 && !b.no_datum && mode != FM_STAGE_B) {
+    Box d{INT_MAX, 0, INT_MAX, 0};
+    const int n = h->ndatum;
+    for (int k = 0; k < n; ++k) {
+      const int i1 = h->datum_tab[k] - 1, i2 = h->datum_tab[k + n] - 1;
+      const int a0 = std::max(i1 - kRad, g.npml), a1 = std::min(i1 + kRad + 1, g.npml + g.n1);
+      const int b0 = std::max(i2 - kRad, g.npml), b1 = std::min(i2 + kRad + 1, g.npml + g.n2);
+      if (a0 >= a1 || b0 >= b1) continue;
+      d.r0 = std::min(d.r0, a0); d.r1 = std::max(d.r1, a1);
+      d.c0 = std::min(d.c0, b0); d.c1 = std::max(d.c1, b1);
+    }
+    if (d.r1 > d.r0) out[1] = d;
+  }
+}
+
+// Columns per CTA with which the batch's runs of `modes` can stay on chip, or
+// 0.  The rule is on the grid (its points fit the SMs' registers and shared
+// memory), on where the stations inject (clear of the rows and columns that
+// are never updated), on how many entries their tables have (they fit beside
+// the fields) and on how much of the grid the gathers read.
+int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> modes) {
+  const Grid& g = h->g;
+  const int RB = g.ld / 64;
+  if (!resident_family(h) || RB > kResRowBlocks || g.npml < 3 || g.n2e < 8) return 0;
+  if (g.ofs == 1 && g.npml % 64 == 0) return 0;  // vz(npml) and vz(npml+1) in different warps
+  const bool fp16 = h->opt.history_fp16 != 0, rho = h->md.rbw1 != nullptr;
+  for (const ShotCtx* c : b.shots)
+    for (int mode : modes) {
+      if (mode == FM_FWD && c->type_src != 0) return 0;
+      Box box[2];
+      gather_boxes(h, b, *c, mode, box);
+      if ((box[0].elems() + box[1].elems()) * sizeof(float) > kRectStepBytes) return 0;
+    }
+  for (int C = std::max(4, (g.n2e + h->sms - 1) / h->sms); C <= kResCols; ++C) {
+    bool ok = true;
+    for (int mode : modes) {
+      int pts = 0, m = 0, nsta = 0;
+      if (mode == FM_FWD || mode == FM_STAGE_A)
+        for (const ShotCtx* c : b.shots) {
+          int p1, m1, n1;
+          if (!resident_heads(g, mode == FM_FWD ? c->srcinfo : c->recinfo, C,
+                              mode == FM_FWD ? 2 : 3, nullptr, &p1, &m1, &n1))
+            return 0;
+          pts = std::max(pts, p1);
+          m = std::max(m, m1);
+          nsta = std::max(nsta, n1);
+        }
+      if (nsta > 60000) return 0;
+      const int occ = resident_occupancy(mode, fp16, rho, RB, resident_smem(C, RB, pts, m, nsta));
+      ok = ok && occ * h->sms >= (g.n2e + C - 1) / C;
+    }
+    if (ok) return C;
+  }
+  return 0;
+}
+
+// Injection tables of a shot's map for C columns per CTA (built once per shot
+// and width).
+void make_tables(daw_handle* h, const ShotCtx& c, const MapInfo& info, const InjMapDev& map, int C,
+                 const char* name, ResTables* t) {
+  if (t->C == C) return;
+  std::vector<int4> heads;
+  ResidentInj d{};
+  resident_heads(h->g, info, C, 2, &heads, &d.pts, &d.m, &d.nsta);
+  const int G = (int)heads.size();
+  if (d.pts > 0) {
+    const std::string p = c.tag + name;
+    int4* head = h->pool.get_t<int4>(p + ".head", G);
+    const size_t n = (size_t)G * d.pts;
+    float* cd = h->pool.get_t<float>(p + ".cd", n * d.m);
+    unsigned short* sta = h->pool.get_t<unsigned short>(p + ".sta", n * d.m);
+    float* kap = h->pool.get_t<float>(p + ".kap", n);
+    upload(head, heads.data(), G * sizeof(int4), h->st);
+    resident_tables(h->g, h->md, map, C, G, head, d.pts, d.m, cd, sta, kap, h->st);
+    check_launch("injection tables");
+    h->tim.kernel_launches += 1;
+    d.head = head; d.cd = cd; d.sta = sta; d.kap = kap;
+  }
+  t->C = C;
+  t->dev = d;
+}
+
+// Decides and prepares the on-chip path for a batch's runs of `modes`; false:
+// the batch runs from global memory.
+bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
+  b.resident = false;
+  b.res_cols = resident_columns(h, b, modes);
+  if (!b.res_cols) return false;
+  try {
+    for (ShotCtx* c : b.shots)
+      for (int mode : modes) {
+        if (mode == FM_FWD) make_tables(h, *c, c->srcinfo, c->srcmap, b.res_cols, "srctab", &c->srctab);
+        if (mode == FM_STAGE_A) make_tables(h, *c, c->recinfo, c->recmap, b.res_cols, "rectab", &c->rectab);
+      }
+  } catch (const DawError& e) {
+    if (e.code != DAW_ERR_OOM) throw;
+    return false;
+  }
+  b.resident = true;
+  return true;
+}
+
+// A pool buffer whose words start at zero (no step tag is zero).
+void* zeroed(daw_handle* h, const std::string& name, size_t bytes) {
+  const bool fresh = h->pool.bufs[name].bytes < bytes;
+  void* p = h->pool.get(name, bytes);
+  if (fresh) CK(cudaMemsetAsync(p, 0, bytes, h->st));
+  return p;
+}
+
+// The time loops of `mode` on chip: the active shots in groups that share a
+// launch, each launch as many steps as its rectangle buffers hold.  With a
+// window (one shot), the window's steps from and to the state in memory.
+void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
+  const Grid& g = h->g;
+  const bool fp16 = h->opt.history_fp16 != 0;
+  const int kmode = mode == FM_STAGE_B_ES ? FM_STAGE_B : mode;
+  ResidentLaunch L{};
+  L.C = b.res_cols;
+  L.G = (g.n2e + L.C - 1) / L.C;
+  L.RB = g.ld / 64;
+  L.slo = mode == FM_STAGE_B_ES ? 1 : 0;
+  L.n1h = hist_ld(h);
+  L.hist_step0 = w && mode != FM_STAGE_A ? w->s0 : 0;
+  L.err = h->d_err;
+  std::vector<ShotCtx*> act;
+  for (ShotCtx* c : b.shots)
+    if (c->active) act.push_back(c);
+  if (act.empty()) return;
+  auto inj_of = [&](const ShotCtx& c) {
+    return mode == FM_FWD ? c.srctab.dev : mode == FM_STAGE_A ? c.rectab.dev : ResidentInj{};
+  };
+  for (const ShotCtx* c : act) {
+    const ResidentInj t = inj_of(*c);
+    L.inj_pts = std::max(L.inj_pts, t.pts);
+    L.inj_m = std::max(L.inj_m, t.m);
+    L.inj_sta = std::max(L.inj_sta, t.nsta);
+  }
+  const int occ = resident_occupancy(kmode, fp16, h->md.rbw1 != nullptr, L.RB,
+                                     resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta));
+  const int room = occ * h->sms / L.G;  // shots whose CTAs are resident together
+  if (room < 1) throw DawError{DAW_ERR_STATE, "on-chip time loop does not fit"};
+  const int q = std::min({room, kResShots, (int)act.size()});
+  h->tim.kernel_family[mode] = 2;
+  h->tim.tile_cols[mode] = L.C;
+  h->tim.ctas_per_sm[mode] = occ;
+  h->tim.ctas_per_sm_v[mode] = 0;
+  h->tim.shots_per_launch[mode] = q;
+  const size_t ctas = (size_t)L.G * q;
+  L.halo = static_cast<ulonglong2*>(
+      zeroed(h, "resident.halo", 4 * ctas * 3 * L.RB * 32 * sizeof(ulonglong2)));
+  L.slots = static_cast<unsigned long long*>(
+      zeroed(h, "resident.slots", 8 * ctas * sizeof(unsigned long long)));
+  for (size_t g0 = 0; g0 < act.size(); g0 += q) {
+    const int n = (int)std::min<size_t>(q, act.size() - g0);
+    L.groups = n;
+    int first = 1, last = 0;
+    size_t rect_elems = 0;
+    std::vector<std::array<Box, 2>> boxes(n);
+    for (int i = 0; i < n; ++i) {
+      ShotCtx& c = *act[g0 + i];
+      last = std::max(last, c.nt);
+      gather_boxes(h, b, c, mode, boxes[i].data());
+      rect_elems += boxes[i][0].elems() + boxes[i][1].elems();
+    }
+    if (w && mode == FM_STAGE_A) last = w->len;
+    if (w && mode != FM_STAGE_A) {
+      first = act[0]->nt - w->s0 - w->len + 1;
+      last = act[0]->nt - w->s0;
+    }
+    const int nsteps = last - first + 1;
+    int chunk = nsteps;
+    float* rect = nullptr;
+    if (rect_elems) {
+      size_t bytes = std::min<size_t>(kRectBytes, rect_elems * sizeof(float) * nsteps);
+      bytes = std::max(bytes, rect_elems * sizeof(float));
+      rect = static_cast<float*>(h->pool.get("resident.rect", bytes));
+      chunk = (int)std::min<size_t>(nsteps, bytes / (rect_elems * sizeof(float)));
+      // launches of similar length
+      chunk = (nsteps + (nsteps + chunk - 1) / chunk - 1) / ((nsteps + chunk - 1) / chunk);
+    }
+    SimClock clk(h);
+    double shot_steps = 0;
+    for (int s0 = first; s0 <= last; s0 += chunk) {
+      const int s1 = std::min(last, s0 + chunk - 1);
+      L.load = w || s0 > first;
+      L.save = w || s1 < last;
+      if (h->res_tag > 0xe0000000u) {  // tags start over
+        CK(cudaMemsetAsync(L.halo, 0, h->pool.bufs["resident.halo"].bytes, h->st));
+        CK(cudaMemsetAsync(L.slots, 0, h->pool.bufs["resident.slots"].bytes, h->st));
+        h->res_tag = 1;
+      }
+      L.tag0 = h->res_tag - (unsigned)s0;
+      h->res_tag += (unsigned)(s1 - s0 + 2);
+      size_t at = 0;
+      for (int i = 0; i < n; ++i) {
+        ShotCtx& c = *act[g0 + i];
+        ResidentShot& S = L.shot[i];
+        S = ResidentShot{};
+        S.px = c.px; S.pz = c.pz; S.vx = c.vx; S.vz = c.vz;
+        S.hist = c.hist;
+        S.amax = c.amax;
+        S.inj = inj_of(c);
+        if (mode == FM_FWD) {
+          S.amp = c.d_s;
+          S.nsta = 1;
+        } else if (mode == FM_STAGE_A) {
+          S.amp = c.d_ampT + (w ? (size_t)w->s0 * c.nr : 0);
+          S.nsta = c.nr;
+        }
+        for (int k = 0; k < 2; ++k) {
+          const Box& x = boxes[i][k];
+          if (!x.elems()) continue;
+          S.rect[k] = ResidentRect{rect + at, rect_elems, x.c1 - x.c0, x.r0, x.r1, x.c0, x.c1};
+          at += x.elems();
+        }
+        if ((mode == FM_FWD || mode == FM_STAGE_B_ES) && c.type_rec == 0) {
+          S.wf = c.d_wf;
+          S.wf_acc = mode == FM_STAGE_B_ES;
+        }
+        S.nt = c.nt;
+        S.first = s0;
+        S.last = w ? s1 : std::min(s1, c.nt);
+        shot_steps += std::max(0, S.last - S.first + 1);
+      }
+      {
+        ResidentOrder& o = resident_order();
+        std::lock_guard<std::mutex> lock(o.mu);
+        auto& e = o.last[h->device];
+        if (!e.first) CK(cudaEventCreateWithFlags(&e.first, cudaEventDisableTiming));
+        if (e.second && e.second != h) CK(cudaStreamWaitEvent(h->st, e.first, 0));
+        CK(resident_launch(g, h->md, L, kmode, fp16, h->st));
+        CK(cudaEventRecord(e.first, h->st));
+        e.second = h;
+      }
+      h->tim.kernel_launches += 1;
+      for (int i = 0; i < n; ++i) {
+        ShotCtx& c = *act[g0 + i];
+        const ResidentShot& S = L.shot[i];
+        const int ns = S.last - S.first + 1;
+        if (S.rect[0].buf) {
+          float* out = mode == FM_FWD ? c.d_datar : c.op_out;
+          const int rev = mode == FM_FWD ? 0 : c.op_reverse;
+          resident_gather(S.rect[0], c.rec, 0, g.n1e, 0, g.n2e, ns, out, c.nt,
+                          rev ? c.nt - S.first : S.first - 1, rev, h->st);
+          h->tim.kernel_launches += 1;
+        }
+        if (S.rect[1].buf) {
+          resident_gather(S.rect[1], h->datum, g.npml, g.npml + g.n1, g.npml, g.npml + g.n2, ns,
+                          mode == FM_FWD ? c.d_redF : c.d_redE, c.nt, S.first - 1, 0, h->st);
+          h->tim.kernel_launches += 1;
+        }
+      }
+      check_launch("on-chip time loop");
+    }
+    double* ms = mode == FM_FWD ? &h->tim.sim_fwd_ms : mode == FM_STAGE_A ? &h->tim.sim_a_ms : &h->tim.sim_b_ms;
+    double* st = mode == FM_FWD ? &h->tim.steps_fwd : mode == FM_STAGE_A ? &h->tim.steps_a : &h->tim.steps_b;
+    (mode == FM_FWD ? h->tim.shot_steps_fwd : mode == FM_STAGE_A ? h->tim.shot_steps_a
+                                                                  : h->tim.shot_steps_b) += shot_steps;
+    clk.stop(ms, st, nsteps, shot_steps);
+    h->tim.point_updates += shot_steps * g.n1e * g.n2e;
+    if (mode != FM_FWD) h->tim.hist_bytes += shot_steps * 3 * g.int_elems() * (fp16 ? 2 : 4);
+  }
+  check_device_error(h);
+}
+
 // Runs `nsteps` steps of `mode`, captured once per batch/mode in a CUDA
 // graph when enabled (kernel arguments are constant; per-shot pointers live in
 // the device-side ShotDevice array, refreshed before each replay).
@@ -868,6 +1238,10 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
 void run_fused(daw_handle* h, Batch& b, int mode, const Window* w = nullptr) {
   const Grid& g = h->g;
   if (w && b.shots.size() != 1) throw DawError{DAW_ERR_STATE, "a windowed run holds one shot"};
+  if (b.resident) {
+    run_resident(h, b, mode, w);
+    return;
+  }
   FusedLaunch L = launch_of(h, b);
   L.persist_v = h->persist_v_mode[mode * 2 + (L.hist_fp16 ? 1 : 0)];
   L.nparam = std::min<int>((int)b.shots.size(), FusedLaunch::kParamShots);
@@ -1034,13 +1408,14 @@ void batch_forward(daw_handle* h, Batch& b) {
       plain_forward(h, *c, c->d_datar, c->d_wf, h->ndatum && !b.no_datum ? c->d_redF : nullptr);
     return;
   }
+  plan_resident(h, b, {FM_FWD});
   for (ShotCtx* c : b.shots) {
     CK(cudaMemsetAsync(c->d_datar, 0, (size_t)c->nt * c->nr * sizeof(float), h->st));
     if (h->ndatum)
       CK(cudaMemsetAsync(c->d_redF, 0, (size_t)c->nt * h->ndatum * sizeof(float), h->st));
-    zero_state(h, *c);
+    if (!b.resident) zero_state(h, *c);
   }
-  fill_shot_devices(h, b, FM_FWD);
+  if (!b.resident) fill_shot_devices(h, b, FM_FWD);
   run_fused(h, b, FM_FWD);
 }
 
@@ -1077,7 +1452,7 @@ void shot_operator_windowed(daw_handle* h, Batch& b, bool esource) {
   auto stage_a = [&](int w) {
     const Window win = window(w);
     CK(cudaMemsetAsync(c.amax, 0, (size_t)(win.len + 1) * 3 * kAmaxSlots * sizeof(unsigned), h->st));
-    fill_shot_devices(h, b, FM_STAGE_A, &win);
+    if (!b.resident) fill_shot_devices(h, b, FM_STAGE_A, &win);
     run_fused(h, b, FM_STAGE_A, &win);
   };
   if (c.nr > 0) {
@@ -1113,7 +1488,7 @@ void shot_operator_windowed(daw_handle* h, Batch& b, bool esource) {
     if (esource && c.d_cost)
       history_cost(c.hist, h->opt.history_fp16, c.amax, win.len, h->g.n1, h->g.n2, hist_ld(h),
                    h->g.npml - h->g.hist_base(), (size_t)hist_ld(h) * h->g.n2, c.d_cost, h->st);
-    fill_shot_devices(h, b, mode, &win);
+    if (!b.resident) fill_shot_devices(h, b, mode, &win);
     run_fused(h, b, mode, &win);
   }
 }
@@ -1134,6 +1509,7 @@ void batch_operator(daw_handle* h, Batch& b, bool esource) {
     }
     return;
   }
+  plan_resident(h, b, {FM_STAGE_A, esource ? FM_STAGE_B_ES : FM_STAGE_B});
   for (ShotCtx* c : b.shots)
     if (c->hist_win > 0) {
       if (b.shots.size() != 1)
@@ -1142,7 +1518,7 @@ void batch_operator(daw_handle* h, Batch& b, bool esource) {
       return;
     }
   for (ShotCtx* c : b.shots) {
-    if (!c->active) continue;
+    if (!c->active || b.resident) continue;
     zero_state(h, *c);
   }
   clear_amax(h, b);
@@ -1151,19 +1527,19 @@ void batch_operator(daw_handle* h, Batch& b, bool esource) {
       transpose_traces(c->op_in, c->d_ampT, c->nt, c->nr, h->st);
       h->tim.kernel_launches += 1;
     }
-  fill_shot_devices(h, b, FM_STAGE_A);
+  if (!b.resident) fill_shot_devices(h, b, FM_STAGE_A);
   run_fused(h, b, FM_STAGE_A);
   for (ShotCtx* c : b.shots) {
     if (!c->active) continue;
     if (esource && c->d_cost)
       history_cost(c->hist, h->opt.history_fp16, c->amax, c->nt, h->g.n1, h->g.n2, hist_ld(h),
                    h->g.npml - h->g.hist_base(), (size_t)hist_ld(h) * h->g.n2, c->d_cost, h->st);
-    zero_state(h, *c);
+    if (!b.resident) zero_state(h, *c);
     CK(cudaMemsetAsync(c->op_out, 0, (size_t)c->nt * c->nr * sizeof(float), h->st));
     if (esource && h->ndatum)
       CK(cudaMemsetAsync(c->d_redE, 0, (size_t)c->nt * h->ndatum * sizeof(float), h->st));
   }
-  fill_shot_devices(h, b, esource ? FM_STAGE_B_ES : FM_STAGE_B);
+  if (!b.resident) fill_shot_devices(h, b, esource ? FM_STAGE_B_ES : FM_STAGE_B);
   run_fused(h, b, esource ? FM_STAGE_B_ES : FM_STAGE_B);
 }
 
@@ -1475,11 +1851,11 @@ void prepare_shot(daw_handle* h, ShotCtx& c, const daw_shot_desc& d, int slot, b
   upload(c.d_s, d.s, (size_t)d.nt * 4, h->st);
   if (d.dobs) upload(c.d_dobs, d.dobs, n * 4, h->st);
   c.rec = make_stations(h, h->pool, p + "rec", d.rec_tab, d.nrec);
-  c.recmap = make_map(h, h->pool, p + "recmap", d.rec_tab, d.nrec);
+  c.recmap = make_map(h, h->pool, p + "recmap", d.rec_tab, d.nrec, &c.recinfo);
   int32_t s5[5];
   std::memcpy(s5, d.src_tab, sizeof s5);
   c.src = make_stations(h, h->pool, p + "src", s5, 1);
-  c.srcmap = make_map(h, h->pool, p + "srcmap", s5, 1);
+  c.srcmap = make_map(h, h->pool, p + "srcmap", s5, 1, &c.srcinfo);
   c.d_wf = want_wf ? h->pool.get_t<float>(p + "wf", g.int_elems() * (size_t)d.nt) : nullptr;
   c.d_ampT = h->pool.get_t<float>(p + "ampT", std::max<size_t>(n, 1));
   // forward-only shots keep no history: one step is allocated so that the
@@ -1674,7 +2050,10 @@ void fetch_outputs(daw_handle* h, ShotCtx& c, daw_shot_out* o) {
 size_t admission_bytes(daw_handle* h) {
   size_t free_b = 0, total_b = 0;
   CK(cudaMemGetInfo(&free_b, &total_b));
-  return (size_t)((double)(free_b + h->pool.total) * 0.92);
+  size_t held = h->pool.total;  // less what the on-chip time loops keep between calls
+  for (const auto& kv : h->pool.bufs)
+    if (kv.first.compare(0, 9, "resident.") == 0) held -= kv.second.bytes;
+  return (size_t)((double)(free_b + held) * 0.92);
 }
 
 // Stage-A history window of a shot of nt steps (fused kernels only): 0 keeps
@@ -1792,7 +2171,7 @@ ShotCtx& single_ctx(daw_handle* h, ShotCtx& c, int nt, const int32_t* ir, int nr
   c.d_redF = a + 7 * n; c.d_redE = c.d_redF + nd; c.d_red = c.d_redE + nd; c.d_redf = c.d_red + nd;
   c.d_s = c.d_redf + nd + nd;
   c.rec = make_stations(h, h->pool, p + "rec", ir, nr);
-  c.recmap = make_map(h, h->pool, p + "recmap", ir, nr);
+  c.recmap = make_map(h, h->pool, p + "recmap", ir, nr, &c.recinfo);
   c.d_wf = want_wf ? h->pool.get_t<float>(p + "wf", h->g.int_elems() * (size_t)nt) : nullptr;
   c.d_ampT = h->pool.get_t<float>(p + "ampT", std::max<size_t>(n, 1));
   const int win = forward_only ? 0 : history_window(h, nt, nr, want_wf, admission_bytes(h));
@@ -2111,7 +2490,7 @@ int daw_submodeling(daw_handle* h, const float* s, int32_t nt, const int32_t* is
     check_table(h, is5, 1, true, "is");
     std::memcpy(c.src5, is5, sizeof c.src5);
     c.src = make_stations(h, h->pool, "shot0.src", is5, 1);
-    c.srcmap = make_map(h, h->pool, "shot0.srcmap", is5, 1);
+    c.srcmap = make_map(h, h->pool, "shot0.srcmap", is5, 1, &c.srcinfo);
     upload(c.d_s, s, (size_t)nt * 4, h->st);
     Batch b;
     b.shots.push_back(&c);

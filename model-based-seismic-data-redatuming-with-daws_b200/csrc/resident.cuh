@@ -1,0 +1,77 @@
+// Time loops on chip (stencil_resident.cu): a shot's whole wavefield stays in
+// the shared and tensor memory of a group of CTAs for all steps of a launch.  This header is what the engine needs to plan and launch them.
+#pragma once
+
+#include "fused.cuh"
+
+namespace daw {
+
+constexpr int kResCols = 27;       // most grid columns per CTA (column masks read 4 ahead)
+constexpr int kResRowBlocks = 15;  // most 64-row blocks (warps) per CTA
+constexpr int kResShots = 16;      // most shots (CTA groups) per launch
+
+// A rectangle of the extended grid whose pressure every step is kept for the
+// Hicks gathers after the loop: rows [r0, r1), columns [c0, c1), step-major
+// [step][row][col] with `ld` columns and `step` elements per step.
+struct ResidentRect {
+  float* buf;
+  size_t step;
+  int ld, r0, r1, c0, c1;
+};
+
+// Injection tables of one station map for CTAs of C columns: CTA b's points
+// are C columns x (rows of its header), `m` entries per point in station
+// order (padded with zero coefficients).
+struct ResidentInj {
+  const int4* head;             // per CTA: first row (even), rows, first station, stations
+  const float* cd;              // coefficient * dt   [cta][pts][m]
+  const unsigned short* sta;    // station - first station of the CTA
+  const float* kap;             // kappa of the point [cta][pts]
+  int pts, m, nsta;             // capacities: points and stations per CTA, entries per point
+};
+
+struct ResidentShot {
+  float *px, *pz, *vx, *vz;     // state at the start (load) and the end (save) of the launch
+  void* hist;
+  unsigned* amax;
+  const float* amp;             // step-major amplitudes [step][nsta]
+  int nsta;
+  ResidentInj inj;              // pts = 0: no injection
+  ResidentRect rect[2];         // buf = nullptr: unused
+  float* wf;                    // optional (n1,n2,nt) pressure output, wf_acc: accumulated
+  int wf_acc;
+  int nt, first, last;          // record length; steps of this launch
+};
+
+struct ResidentLaunch {
+  int C, G, RB, groups;         // columns per CTA, CTAs per shot, row blocks, shots
+  ulonglong2* halo;             // [phase][parity][cta][3][RB * 32]
+  unsigned long long* slots;    // [ring of 4][field][cta] (max bits, tag)
+  unsigned tag0;                // step tags of this launch: tag0 + step
+  int load, save;               // state from / to global memory (else zero / dropped)
+  int slo;                      // pressure source margin (1: final esource)
+  int n1h, hist_step0;
+  int inj_pts, inj_m, inj_sta;  // shared-memory capacities of the injection tables
+  unsigned* err;
+  unsigned long long nz;        // (-0, -0), set by resident_launch
+  ResidentShot shot[kResShots];
+};
+
+// Dynamic shared memory of a CTA.
+size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta);
+// CTAs per SM of (mode, fp16, density) with that much shared memory; 0 when it does not fit.
+int resident_occupancy(int mode, bool fp16, bool rho, int RB, size_t smem);
+cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaunch& L, int mode,
+                            bool fp16, cudaStream_t st);
+// Fills the injection tables of a station map for the CTAs' headers.
+void resident_tables(const Grid& g, const ModelDev& m, const InjMapDev& map, int C, int G,
+                     const int4* head, int pts, int mm, float* cd, unsigned short* sta, float* kap,
+                     cudaStream_t st);
+// Hicks sums of a station set for steps 0 .. nsteps-1 of a rectangle buffer,
+// the support clipped to rows [lo1, hi1) and columns [lo2, hi2):
+// out[row(step) + nt * station], row = row0 + step, or row0 - step when reverse.
+void resident_gather(const ResidentRect& r, const StationsDev& st, int lo1, int hi1, int lo2,
+                     int hi2, int nsteps, float* out, int nt, int row0, int reverse,
+                     cudaStream_t s);
+
+}  // namespace daw
