@@ -938,8 +938,8 @@ bool resident_heads(const Grid& g, const MapInfo& info, int C, int off, std::vec
       *m = std::max(*m, info.cnt[c]);
     }
     if (hi < lo) continue;
-    lo &= ~1;
-    const int rows = (hi | 1) - lo + 1;
+    lo &= ~3;
+    const int rows = (hi | 3) - lo + 1;
     if (heads) (*heads)[b] = make_int4(lo, rows, s0, s1 - s0 + 1);
     *pts = std::max(*pts, C * rows);
     *nsta = std::max(*nsta, s1 - s0 + 1);
@@ -981,9 +981,9 @@ void gather_boxes(const daw_handle* h, const Batch& b, const ShotCtx& c, int mod
 // the fields) and on how much of the grid the gathers read.
 int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> modes) {
   const Grid& g = h->g;
-  const int RB = g.ld / 64;
+  const int RB = (g.n1e + 127) / 128;
   if (!resident_family(h) || RB > kResRowBlocks || g.npml < 3 || g.n2e < 8) return 0;
-  if (g.ofs == 1 && g.npml % 64 == 0) return 0;  // vz(npml) and vz(npml+1) in different warps
+  if (g.ofs == 1 && g.npml % 128 == 0) return 0;  // vz(npml) and vz(npml+1) in different warps
   const bool fp16 = h->opt.history_fp16 != 0, rho = h->md.rbw1 != nullptr;
   for (const ShotCtx* c : b.shots)
     for (int mode : modes) {
@@ -1007,7 +1007,7 @@ int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> m
           nsta = std::max(nsta, n1);
         }
       if (nsta > 60000) return 0;
-      const int occ = resident_occupancy(mode, fp16, rho, RB, resident_smem(C, RB, pts, m, nsta));
+      const int occ = resident_occupancy(mode, fp16, rho, C, RB, resident_smem(C, RB, pts, m, nsta));
       ok = ok && occ * h->sms >= (g.n2e + C - 1) / C;
     }
     if (ok) return C;
@@ -1079,7 +1079,7 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
   ResidentLaunch L{};
   L.C = b.res_cols;
   L.G = (g.n2e + L.C - 1) / L.C;
-  L.RB = g.ld / 64;
+  L.RB = (g.n1e + 127) / 128;
   L.slo = mode == FM_STAGE_B_ES ? 1 : 0;
   L.n1h = hist_ld(h);
   L.hist_step0 = w && mode != FM_STAGE_A ? w->s0 : 0;
@@ -1097,7 +1097,7 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
     L.inj_m = std::max(L.inj_m, t.m);
     L.inj_sta = std::max(L.inj_sta, t.nsta);
   }
-  const int occ = resident_occupancy(kmode, fp16, h->md.rbw1 != nullptr, L.RB,
+  const int occ = resident_occupancy(kmode, fp16, h->md.rbw1 != nullptr, L.C, L.RB,
                                      resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta));
   const int room = occ * h->sms / L.G;  // shots whose CTAs are resident together
   if (room < 1) throw DawError{DAW_ERR_STATE, "on-chip time loop does not fit"};
@@ -1109,7 +1109,7 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
   h->tim.shots_per_launch[mode] = q;
   const size_t ctas = (size_t)L.G * q;
   L.halo = static_cast<ulonglong2*>(
-      zeroed(h, "resident.halo", 4 * ctas * 3 * L.RB * 32 * sizeof(ulonglong2)));
+      zeroed(h, "resident.halo", 4 * ctas * 3 * L.RB * 64 * sizeof(ulonglong2)));
   L.slots = static_cast<unsigned long long*>(
       zeroed(h, "resident.slots", 8 * ctas * sizeof(unsigned long long)));
   for (size_t g0 = 0; g0 < act.size(); g0 += q) {

@@ -7,7 +7,8 @@
 namespace daw {
 
 constexpr int kResCols = 27;       // most grid columns per CTA (column masks read 4 ahead)
-constexpr int kResRowBlocks = 15;  // most 64-row blocks (warps) per CTA
+constexpr int kResRowBlocks = 15;  // most 128-row blocks per CTA
+constexpr int kResWarps = 16;      // most warps per CTA (128 registers a thread)
 constexpr int kResShots = 16;      // most shots (CTA groups) per launch
 
 // A rectangle of the extended grid whose pressure every step is kept for the
@@ -23,7 +24,7 @@ struct ResidentRect {
 // are C columns x (rows of its header), `m` entries per point in station
 // order (padded with zero coefficients).
 struct ResidentInj {
-  const int4* head;             // per CTA: first row (even), rows, first station, stations
+  const int4* head;             // per CTA: first row (of 4), rows, first station, stations
   const float* cd;              // coefficient * dt   [cta][pts][m]
   const unsigned short* sta;    // station - first station of the CTA
   const float* kap;             // kappa of the point [cta][pts]
@@ -44,8 +45,9 @@ struct ResidentShot {
 };
 
 struct ResidentLaunch {
-  int C, G, RB, groups;         // columns per CTA, CTAs per shot, row blocks, shots
-  ulonglong2* halo;             // [phase][parity][cta][3][RB * 32]
+  int C, G, RB, groups;         // columns per CTA, CTAs per shot, 128-row blocks, shots
+  int CG, CW;                   // column groups and columns of a group (resident_launch)
+  ulonglong2* halo;             // [phase][parity][cta][3][RB * 32][2]
   unsigned long long* slots;    // [ring of 4][field][cta] (max bits, tag)
   unsigned tag0;                // step tags of this launch: tag0 + step
   int load, save;               // state from / to global memory (else zero / dropped)
@@ -59,8 +61,10 @@ struct ResidentLaunch {
 
 // Dynamic shared memory of a CTA.
 size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta);
+// Warps of a CTA: column groups and columns per group.
+void resident_groups(int C, int RB, int* cg, int* cw);
 // CTAs per SM of (mode, fp16, density) with that much shared memory; 0 when it does not fit.
-int resident_occupancy(int mode, bool fp16, bool rho, int RB, size_t smem);
+int resident_occupancy(int mode, bool fp16, bool rho, int C, int RB, size_t smem);
 cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaunch& L, int mode,
                             bool fp16, cudaStream_t st);
 // Fills the injection tables of a station map for the CTAs' headers.

@@ -2,18 +2,20 @@
 //
 // One cooperative launch runs all steps of a time loop (or a long chunk of
 // them) with the wavefield held on chip: a group of G CTAs owns one shot, CTA
-// b the grid columns [b C, b C + C) over all rows.  A compute warp owns 64 rows of
-// them, a lane two adjacent rows: px and pz of the lane's 2 x C points are in
-// tensor memory (used as a scratchpad a warp reads and writes by column), vx, vz
-// and kappa in shared memory.  What one step moves is then the history stream
-// and three halo columns per CTA and half step, not the state.
+// b the grid columns [b C, b C + C) over all rows.  A compute warp owns 128 rows
+// of some of them (the CTA's columns are split over column groups of warps), a
+// lane four adjacent rows: px, pz and kappa are in tensor memory, used as a
+// scratchpad that a warp reads and writes by column, vx and vz in shared memory.
+// What one step moves is then the history stream and three halo columns per CTA
+// and half step, not the state.
 //
 // Halo columns go from lane to lane of neighbouring CTAs through L2: the
 // writer stores (value, step tag) as one 64-bit word, so the reader's poll of
 // the data is also the wait and no fence or flag follows it.  A lane needs its
-// neighbour CTA's values of its own two rows only, and only for the first two
-// and the last column; those columns are computed last in a half step, so the
-// words travel while the columns between are computed.  Buffers alternate by
+// neighbour CTA's values of its own rows only, and only for the first two and
+// the last column; those columns are computed last in a half step, so the
+// words travel while the columns between are computed, and they are fetched
+// into shared memory a few columns ahead of their use.  Buffers alternate by
 // step parity: a CTA writes parity s only after it has read its neighbours'
 // words of step s - 1, which they store after their last read of step s - 2.
 // Rows couple neighbouring warps (vz through shared memory, p through warp
@@ -22,13 +24,14 @@
 // Stage A stores its FP16 histories with one scale per step and field, taken
 // from the maximum over the whole grid.  An extra warp per CTA exchanges the
 // CTAs' maxima through tagged words during the half step after a field is
-// complete, and the history of step s is stored from the registers and shared
+// complete, and the history of step s is stored from the tensor and shared
 // memory in step s + 1, just before the values are updated (the last step's
 // after the loop).
 //
 // Rows 0, 1 and the last rows and columns are never updated and the caller
 // keeps sources away from them, so they stay zero: their update coefficients
-// are set to zero instead of branching.
+// are set to zero instead of branching.  The same holds for px and pz above the
+// free surface, where the pressure is zeroed.
 //
 // Arithmetic: the reference's separately rounded FP32 operations, two rows at
 // a time in packed (f32x2) instructions; bit-identical to the other kernels.
@@ -36,15 +39,17 @@
 // Every wait is bounded: after its limit it raises kErrTimeout, and the other
 // waits of the grid see the flag and stop waiting too.
 //
-// What bounds it: instruction issue (about 230 warp instructions per 64 points
-// and step of stage A, 111 of them arithmetic or memory) for wide CTAs, the
-// exchange latency (about 1.5 us per half step) for narrow ones.  The fields
-// are not in registers because their columns must then be unrolled: that
-// version ran out of the instruction cache (30 us against 14).
+// What bounds it: for wide CTAs instruction issue and the latency between
+// dependent instructions (16 warps an SM is what 128 registers allow; about 150
+// instructions per lane quad and half step, 46 of them arithmetic), for narrow
+// ones the exchange latency (about 0.5 us per half step).  Tried and slower: the fields in
+// registers with all columns unrolled (30 us a step against 14: instruction
+// cache), lanes of two rows (13.2-14.0 us against 9.2-12.5: the same number of
+// instructions per lane), a separate copy of the column code for the edges.
 // Measured per shot step against the split kernels (B200, FP16 histories):
-// 751 x 2301 (17 columns a CTA) forward 13.2 us against 20.1, stage A 14.0
-// against 20.7-23.0, stage B 13.8 against 19.7-24.7; 151 x 461 (4 columns)
-// 4.1-6.2 us against 12-15.
+// 751 x 2301 (17 columns a CTA) forward 9.2 us against 20.1, stage A 12.5
+// against 20.7-23.0, stage B 9.7 against 19.7-24.7; 151 x 461 (4 columns)
+// 2.4-6.2 us against 12-15.
 #include "resident.cuh"
 #include "tma.cuh"
 
@@ -84,11 +89,36 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
 }
 constexpr u64 kNegZero2 = 0x8000000080000000ull;
 
-// (value, tag) words
-__device__ __forceinline__ void ll_store(ulonglong2* p, u64 v, unsigned tag) {
-  const float2 f = up(v);
-  const u64 a = (u64)tag << 32 | __float_as_uint(f.x), b = (u64)tag << 32 | __float_as_uint(f.y);
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+// Four rows of a lane.
+struct Q4 {
+  u64 a, b;  // rows 0-1, 2-3
+};
+__device__ __forceinline__ Q4 add4(Q4 x, Q4 y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ Q4 sub4(Q4 x, Q4 y) { return {sub2(x.a, y.a), sub2(x.b, y.b)}; }
+__device__ __forceinline__ Q4 lds4(const Q4* p) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  return {v.x, v.y};
+}
+__device__ __forceinline__ void sts4(Q4* p, Q4 v) {
+  *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.a, v.b);
+}
+__device__ __forceinline__ Q4 pk4(float x, float y, float z, float w) { return {pk(x, y), pk(z, w)}; }
+__device__ __forceinline__ float4 up4(Q4 v) {
+  const float2 a = up(v.a), b = up(v.b);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+constexpr Q4 kZero4{0ull, 0ull};
+
+// (value, tag) words: a lane's four rows are four of them, in two 16-byte halves.
+__device__ __forceinline__ void ll_store(ulonglong2* p, Q4 v, unsigned tag) {
+  const float4 f = up4(v);
+  const u64 t = (u64)tag << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p),
+               "l"(t | __float_as_uint(f.x)), "l"(t | __float_as_uint(f.y))
+               : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p + 1),
+               "l"(t | __float_as_uint(f.z)), "l"(t | __float_as_uint(f.w))
+               : "memory");
 }
 __device__ __forceinline__ ulonglong2 ll_load(const ulonglong2* p) {
   ulonglong2 v;
@@ -120,27 +150,36 @@ struct Poll {
   }
 };
 
-__device__ __forceinline__ u64 ll_wait1(const ulonglong2* p, unsigned tag, Poll& w) {
-  ulonglong2 a = ll_load(p);
-  for (int n = 0; !w.dead; ++n) {
-    const bool ok = (unsigned)(a.x >> 32) == tag && (unsigned)(a.y >> 32) == tag;
-    if (__all_sync(kAll, ok) || w.give_up(n)) break;
-    a = ll_load(p);
-  }
-  return (a.y << 32) | (a.x & 0xffffffffu);
+// N halo columns at p, p + stride, ...: `fetch` copies the lane's words to its
+// place in shared memory, early and without waiting; `get` checks their tags
+// there and polls the words themselves until all carry the tag.
+template <int N>
+__device__ __forceinline__ void halo_fetch(ulonglong2* sh, const ulonglong2* p, size_t stride) {
+#pragma unroll
+  for (int k = 0; k < 2 * N; ++k)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(sh + (k / 2) * 64 + (k & 1))),
+                 "l"(p + (k / 2) * stride + (k & 1))
+                 : "memory");
 }
-__device__ __forceinline__ void ll_wait2(const ulonglong2* p, const ulonglong2* q, unsigned tag,
-                                         Poll& w, u64& vp, u64& vq) {
-  ulonglong2 a = ll_load(p), b = ll_load(q);
-  for (int n = 0; !w.dead; ++n) {
-    const bool ok = (unsigned)(a.x >> 32) == tag && (unsigned)(a.y >> 32) == tag &&
-                    (unsigned)(b.x >> 32) == tag && (unsigned)(b.y >> 32) == tag;
-    if (__all_sync(kAll, ok) || w.give_up(n)) break;
-    a = ll_load(p);
-    b = ll_load(q);
+template <int N>
+__device__ __forceinline__ void halo_get(const ulonglong2* sh, const ulonglong2* p, size_t stride,
+                                         unsigned tag, Poll& w, Q4 (&v)[N]) {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  ulonglong2 x[2 * N];
+#pragma unroll
+  for (int k = 0; k < 2 * N; ++k) x[k] = sh[(k / 2) * 64 + (k & 1)];
+  for (int n = 0;; ++n) {
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 2 * N; ++k)
+      ok = ok && (unsigned)(x[k].x >> 32) == tag && (unsigned)(x[k].y >> 32) == tag;
+    if (w.dead || __all_sync(kAll, ok) || w.give_up(n)) break;
+#pragma unroll
+    for (int k = 0; k < 2 * N; ++k) x[k] = ll_load(p + (k / 2) * stride + (k & 1));
   }
-  vp = (a.y << 32) | (a.x & 0xffffffffu);
-  vq = (b.y << 32) | (b.x & 0xffffffffu);
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    v[k] = {(x[2 * k].y << 32) | (unsigned)x[2 * k].x, (x[2 * k + 1].y << 32) | (unsigned)x[2 * k + 1].x};
 }
 
 // Maximum of the group's tagged words at `s` (G of them), by one warp.
@@ -157,6 +196,7 @@ __device__ __forceinline__ unsigned group_max(const u64* s, int G, unsigned tag,
         ok = ok && (unsigned)(v[k] >> 32) == tag;
       }
       if (w.dead || __all_sync(kAll, ok) || w.give_up(n)) break;
+      __nanosleep(100);  // leaves the issue slots to the other warps
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) m = max(m, (unsigned)v[k]);
@@ -164,93 +204,89 @@ __device__ __forceinline__ unsigned group_max(const u64* s, int G, unsigned tag,
   return __reduce_max_sync(kAll, m);
 }
 
-// A history row pair: FP16 in 32 bits, FP32 in 64.  Loads and stores are
-// predicated (a load that is off gives 0), so that they cost no branch.
+// The history of a lane's four rows: FP16 in 64 bits, FP32 in 128.  Loads and
+// stores are predicated (a load that is off gives 0), so that they cost no branch.
 template <bool FP16>
-struct HPair;
+struct HQuad;
 template <>
-struct HPair<true> {
-  typedef uint32_t T;
+struct HQuad<true> {
+  typedef uint2 T;
   static __device__ __forceinline__ T load(const char* p, unsigned on) {
     T v;
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.b32 %0, 0;\n"
-        " @p ld.global.nc.L1::no_allocate.b32 %0, [%1];\n}"
-        : "=&r"(v)
+        "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n mov.b32 %0, 0;\n mov.b32 %1, 0;\n"
+        " @p ld.global.nc.L1::no_allocate.v2.b32 {%0, %1}, [%2];\n}"
+        : "=&r"(v.x), "=&r"(v.y)
         : "l"(p), "r"(on));
     return v;
   }
-  static __device__ __forceinline__ u64 get(T v) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
-    return pk(f.x, f.y);
+  static __device__ __forceinline__ Q4 get(T v) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&v.x));
+    const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&v.y));
+    return {pk(a.x, a.y), pk(b.x, b.y)};
   }
-  static __device__ __forceinline__ void put(char* p, u64 v, uint64_t pol, unsigned on) {
-    const float2 f = up(v);
-    const __half2 q = __floats2half2_rn(f.x, f.y);
+  static __device__ __forceinline__ void put(char* p, Q4 v, uint64_t pol, unsigned on) {
+    const float4 f = up4(v);
+    const __half2 a = __floats2half2_rn(f.x, f.y), b = __floats2half2_rn(f.z, f.w);
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n"
-        " @p st.global.L2::cache_hint.b32 [%0], %1, %2;\n}" ::"l"(p),
-        "r"(*reinterpret_cast<const uint32_t*>(&q)), "l"(pol), "r"(on)
-        : "memory");
-  }
-  static __device__ __forceinline__ void put2(char* p, u64 v, char* p2, u64 v2, uint64_t pol,
-                                              unsigned on) {
-    const float2 f = up(v), f2 = up(v2);
-    const __half2 q = __floats2half2_rn(f.x, f.y), q2 = __floats2half2_rn(f2.x, f2.y);
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %5, 0;\n"
-        " @p st.global.L2::cache_hint.b32 [%0], %1, %4;\n"
-        " @p st.global.L2::cache_hint.b32 [%2], %3, %4;\n}" ::"l"(p),
-        "r"(*reinterpret_cast<const uint32_t*>(&q)), "l"(p2),
-        "r"(*reinterpret_cast<const uint32_t*>(&q2)), "l"(pol), "r"(on)
+        "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+        " @p st.global.L2::cache_hint.v2.b32 [%0], {%1, %2}, %3;\n}" ::"l"(p),
+        "r"(*reinterpret_cast<const uint32_t*>(&a)), "r"(*reinterpret_cast<const uint32_t*>(&b)),
+        "l"(pol), "r"(on)
         : "memory");
   }
 };
 template <>
-struct HPair<false> {
-  typedef u64 T;
+struct HQuad<false> {
+  typedef ulonglong2 T;
   static __device__ __forceinline__ T load(const char* p, unsigned on) {
     T v;
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n mov.b64 %0, 0;\n"
-        " @p ld.global.nc.L1::no_allocate.b64 %0, [%1];\n}"
-        : "=&l"(v)
+        "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n mov.b64 %0, 0;\n mov.b64 %1, 0;\n"
+        " @p ld.global.nc.L1::no_allocate.v2.b64 {%0, %1}, [%2];\n}"
+        : "=&l"(v.x), "=&l"(v.y)
         : "l"(p), "r"(on));
     return v;
   }
-  static __device__ __forceinline__ u64 get(T v) { return v; }
-  static __device__ __forceinline__ void put(char* p, u64 v, uint64_t pol, unsigned on) {
+  static __device__ __forceinline__ Q4 get(T v) { return {v.x, v.y}; }
+  static __device__ __forceinline__ void put(char* p, Q4 v, uint64_t pol, unsigned on) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n"
-        " @p st.global.L2::cache_hint.b64 [%0], %1, %2;\n}" ::"l"(p),
-        "l"(v), "l"(pol), "r"(on)
+        "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+        " @p st.global.L2::cache_hint.v2.b64 [%0], {%1, %2}, %3;\n}" ::"l"(p),
+        "l"(v.a), "l"(v.b), "l"(pol), "r"(on)
         : "memory");
-  }
-  static __device__ __forceinline__ void put2(char* p, u64 v, char* p2, u64 v2, uint64_t pol,
-                                              unsigned on) {
-    put(p, v, pol, on);
-    put(p2, v2, pol, on);
   }
 };
 
 // Predicated shared-memory accesses.
-__device__ __forceinline__ void sts_if(u64* p, u64 v, bool on) {
+__device__ __forceinline__ void sts_if(u64* p, u64 v, unsigned on) {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p st.shared.b64 [%0], %1;\n}" ::"r"(
                    smem_u32(p)),
-               "l"(v), "r"((unsigned)on)
+               "l"(v), "r"(on)
                : "memory");
 }
-__device__ __forceinline__ void lds_if(float& v, const float* p, bool on) {
+__device__ __forceinline__ void lds_if(float& v, const float* p, unsigned on) {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.shared.f32 %0, [%1];\n}"
                : "+f"(v)
-               : "r"(smem_u32(p)), "r"((unsigned)on)
-               : "memory");
+               : "r"(smem_u32(p)), "r"(on));
 }
-__device__ __forceinline__ void lds_if(float& x, float& y, const float* p, bool on) {
+__device__ __forceinline__ void lds_if(float& x, float& y, const float* p, unsigned on) {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.shared.v2.f32 {%0, %1}, [%2];\n}"
                : "+f"(x), "+f"(y)
-               : "r"(smem_u32(p)), "r"((unsigned)on)
-               : "memory");
+               : "r"(smem_u32(p)), "r"(on));
+}
+// Four rows `ld` floats apart, each where its bit is set.
+__device__ __forceinline__ void stg_rows(float* p, int ld, float4 v, unsigned rows) {
+  asm volatile(
+      "{\n .reg .pred p, q, r, s;\n .reg .b64 a, d;\n .reg .b32 t;\n"
+      " and.b32 t, %6, 1;\n setp.ne.u32 p, t, 0;\n and.b32 t, %6, 2;\n setp.ne.u32 q, t, 0;\n"
+      " and.b32 t, %6, 4;\n setp.ne.u32 r, t, 0;\n and.b32 t, %6, 8;\n setp.ne.u32 s, t, 0;\n"
+      " mul.wide.s32 d, %1, 4;\n"
+      " @p st.global.f32 [%0], %2;\n add.s64 a, %0, d;\n @q st.global.f32 [a], %3;\n"
+      " add.s64 a, a, d;\n @r st.global.f32 [a], %4;\n add.s64 a, a, d;\n"
+      " @s st.global.f32 [a], %5;\n}" ::"l"(p),
+      "r"(ld), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(rows)
+      : "memory");
 }
 
 __device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes) {
@@ -258,32 +294,57 @@ __device__ __forceinline__ void l2_prefetch(const void* p, unsigned bytes) {
 }
 
 // Tensor memory as a scratchpad: 32-bit columns of 32 lanes per warp quadrant.
-// A warp reaches the lanes of its quadrant (warp % 4) only.
-__device__ __forceinline__ void tm_ld4(unsigned a, unsigned (&r)[4]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(a));
+// A warp reaches the lanes of its quadrant (warp % 4) only.  A record is a
+// lane's px and pz (8 words) and kappa (4 words) of one grid column.
+__device__ __forceinline__ void tm_ld(unsigned a, Q4& x, Q4& z) {
+  asm volatile(
+      "{\n .reg .b32 r0, r1, r2, r3, r4, r5, r6, r7;\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0, r1, r2, r3, r4, r5, r6, r7}, [%4];\n"
+      " tcgen05.wait::ld.sync.aligned;\n"
+      " mov.b64 %0, {r0, r1};\n mov.b64 %1, {r2, r3};\n mov.b64 %2, {r4, r5};\n mov.b64 %3, {r6, r7};\n}"
+      : "=l"(x.a), "=l"(x.b), "=l"(z.a), "=l"(z.b)
+      : "r"(a));
 }
-// The loads' registers are read after this wait only (they are its operands).
-__device__ __forceinline__ void tm_wait(unsigned (&r)[4]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])::"memory");
+// the same with kappa's record at k
+__device__ __forceinline__ void tm_ld(unsigned a, unsigned k, Q4& x, Q4& z, Q4& q) {
+  asm volatile(
+      "{\n .reg .b32 r0, r1, r2, r3, r4, r5, r6, r7, q0, q1, q2, q3;\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {r0, r1, r2, r3, r4, r5, r6, r7}, [%6];\n"
+      " tcgen05.ld.sync.aligned.32x32b.x4.b32 {q0, q1, q2, q3}, [%7];\n"
+      " tcgen05.wait::ld.sync.aligned;\n"
+      " mov.b64 %0, {r0, r1};\n mov.b64 %1, {r2, r3};\n mov.b64 %2, {r4, r5};\n mov.b64 %3, {r6, r7};\n"
+      " mov.b64 %4, {q0, q1};\n mov.b64 %5, {q2, q3};\n}"
+      : "=l"(x.a), "=l"(x.b), "=l"(z.a), "=l"(z.b), "=l"(q.a), "=l"(q.b)
+      : "r"(a), "r"(k));
 }
-__device__ __forceinline__ void tm_st4(unsigned a, u64 x, u64 z) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a),
-               "r"((unsigned)x), "r"((unsigned)(x >> 32)), "r"((unsigned)z), "r"((unsigned)(z >> 32))
-               : "memory");
+__device__ __forceinline__ void tm_st(unsigned a, Q4 x, Q4 z) {
+  asm volatile(
+      "{\n .reg .b32 r0, r1, r2, r3, r4, r5, r6, r7;\n"
+      " mov.b64 {r0, r1}, %1;\n mov.b64 {r2, r3}, %2;\n mov.b64 {r4, r5}, %3;\n mov.b64 {r6, r7}, %4;\n"
+      " tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {r0, r1, r2, r3, r4, r5, r6, r7};\n}" ::"r"(a),
+      "l"(x.a), "l"(x.b), "l"(z.a), "l"(z.b)
+      : "memory");
+}
+__device__ __forceinline__ void tm_st(unsigned a, Q4 x) {
+  asm volatile(
+      "{\n .reg .b32 r0, r1, r2, r3;\n mov.b64 {r0, r1}, %1;\n mov.b64 {r2, r3}, %2;\n"
+      " tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {r0, r1, r2, r3};\n}" ::"r"(a),
+      "l"(x.a), "l"(x.b)
+      : "memory");
 }
 __device__ __forceinline__ void tm_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ u64 pku(unsigned x, unsigned y) {
-  return pk(__uint_as_float(x), __uint_as_float(y));
+// The CTA barrier, which also orders tensor-memory accesses of different warps.
+__device__ __forceinline__ void sync_cta() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
 // Shared-memory layout (offsets in bytes, 16-byte aligned sections).
 struct Lay {
-  int fld, edge, col, row, tcd, term, tsta, tkap, amp, misc, total;
+  int fld, halo, edge, col, row, tcd, term, tsta, tkap, amp, misc, total;
 };
 __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta) {
   Lay l;
@@ -293,10 +354,13 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta) {
     o += (bytes + 15) / 16 * 16;
     return at;
   };
-  l.fld = take(RB * C * 768);        // [warp][column][vx, vz, kappa][lane]
-  l.edge = take((RB + 2) * C * 16);  // [warp + 1][column][first, last pair of p]
+  // [row block][column -2 .. C][vx, vz][lane] quads; columns -2, -1 and C hold
+  // the neighbours' vx
+  l.fld = take(RB * (C + 3) * 1024);
+  l.halo = take(RB * 4096);          // [row block][2 left, 2 right columns][lane][2] halo words
+  l.edge = take((RB + 2) * C * 16);  // [row block + 1][column][first, last pair of p]
   l.col = take(C * 32);              // [column][d2a, d2a, d2a1, d2a1, d2b, d2b, bw2, bw2]
-  l.row = take(5 * RB * 32 * 8);
+  l.row = take(4 * RB * 512);        // d1a, d1a1, d1b, bw1
   l.tcd = take(pts * m * 4);
   l.term = take(pts * m * 4);
   l.tsta = take(pts * m * 2);
@@ -306,24 +370,34 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta) {
   l.total = o;
   return l;
 }
-// Tensor-memory columns: px, pz (4 words a grid column and warp of the quadrant).
-__host__ __device__ inline int tm_words(int C, int RB) { return (RB + 3) / 4 * C * 4; }
+// Tensor-memory columns per row block of a quadrant: px, pz of the grid columns
+// -1 .. C + 1 (those outside 0 .. C - 1 hold the neighbours' p), kappa of 0 .. C - 1.
+__host__ __device__ inline int tm_words(int C, int RB) { return (RB + 3) / 4 * ((C + 3) * 8 + C * 4); }
 __host__ __device__ inline int tm_alloc(int C, int RB) {
   int n = 32;
   while (n < tm_words(C, RB)) n *= 2;
   return n;
 }
+// Warps: CG column groups of RB row blocks, the groups a multiple of 4 warps
+// apart (a row block's warps share a quadrant), and the extra warp in a gap or
+// at the end.
+__host__ __device__ inline int group_warps(int RB) { return (RB + 3) / 4 * 4; }
+__host__ __device__ inline int cta_warps(int RB, int CG) {
+  return RB % 4 ? CG * group_warps(RB) : CG * group_warps(RB) + 1;
+}
+__host__ __device__ inline int aux_warp(int RB, int CG) {
+  return RB % 4 ? RB : CG * group_warps(RB);
+}
 
-// The injection terms ((c dt) amp) kappa of one step, by the compute warps.
-__device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int pts, int m,
-                                          int nthreads) {
+// The injection terms ((c dt) amp) kappa of one step, by all warps.
+__device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int pts, int m) {
   const float2* cd = reinterpret_cast<const float2*>(sm + l.tcd);
   float2* term = reinterpret_cast<float2*>(sm + l.term);
   const ushort2* sta = reinterpret_cast<const ushort2*>(sm + l.tsta);
   const float* kap = reinterpret_cast<const float*>(sm + l.tkap);
   const float* amp = reinterpret_cast<const float*>(sm + l.amp);
   const int mh = m / 2;
-  for (int p = threadIdx.x; p < pts; p += nthreads) {
+  for (int p = threadIdx.x; p < pts; p += blockDim.x) {
     const float kv = kap[p];
     for (int k = 0; k < mh; ++k) {
       const float2 c = cd[p * mh + k];
@@ -334,44 +408,49 @@ __device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int p
 }
 
 template <int MODE, bool FP16, bool RHO>
-__global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
+__global__ void __launch_bounds__(32 * kResWarps, 1)
     k_resident(const __grid_constant__ Grid g, const __grid_constant__ ModelDev md,
                const __grid_constant__ ResidentLaunch L) {
   constexpr bool kA = MODE == FM_STAGE_A, kB = MODE == FM_STAGE_B, kF = MODE == FM_FWD;
-  constexpr int U = 4;  // columns per loop iteration
-  using HP = HPair<FP16>;
-  using HT = typename HP::T;
+  constexpr int FS = 64;  // quads between a lane's columns
+  constexpr int HR = 2;   // history columns read ahead
+  using HQ = HQuad<FP16>;
+  using HT = typename HQ::T;
   extern __shared__ __align__(16) unsigned char sm[];
   const int C = L.C, G = L.G, RB = L.RB;
   const Lay l = layout(C, RB, L.inj_pts, L.inj_m, L.inj_sta);
   const int grp = blockIdx.x / G, b = blockIdx.x - grp * G;
   const ResidentShot& S = L.shot[grp];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ncomp = RB * 32;            // compute threads
-  const bool aux = warp == RB;          // the extra warp
-  const int c0 = b * C, i1 = 64 * warp + 2 * lane;
+  // the warp index from a shuffle: the compiler then knows that it, and all
+  // control that follows from it, is uniform over the warp
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(kAll, tid >> 5, 0);
+  const int rb = warp % group_warps(RB), cg = warp / group_warps(RB);  // row block, column group
+  const bool aux = warp == aux_warp(RB, L.CG);
+  const bool comp = !aux && rb < RB && cg < L.CG;  // else an idle warp: barriers only
+  const int c0 = b * C, i1 = 128 * rb + 4 * lane;
   const int npml = g.npml, ld = g.ld;
   const int first = S.first, last = S.last;
   if (first > last) return;             // uniform over the group
-  // the lane's vx, vz, kappa of column j: F[96 j], F[96 j + 32], F[96 j + 64];
-  // the vz pairs above and below it at FU, FD (lanes 0 and 31: in the
-  // neighbouring warps' areas; the grid's first and last pair, which are never
+  const int clo = cg * L.CW, chi = min(C, clo + L.CW);  // the warp's columns
+  // the lane's vx, vz of column j: F[FS j], F[FS j + 32]; the vz pair above and the row below it at FU, FD (lanes 0 and 31: in the
+  // neighbouring row blocks; the grid's first and last rows, which are never
   // updated, stand for the zeros beyond them)
-  u64* const F = reinterpret_cast<u64*>(sm + l.fld) + warp * C * 96 + lane;
-  const u64* const FU = F + 32 + (lane > 0 ? -1 : warp > 0 ? 31 - C * 96 : 0);
-  const u64* const FD = F + 32 + (lane < 31 ? 1 : warp < RB - 1 ? C * 96 - 31 : 0);
-  u64* const ED = reinterpret_cast<u64*>(sm + l.edge) + (warp + 1) * C * 2;
-  u64* const EDL = ED + (lane == 31);  // where lanes 0 and 31 put their pairs
-  const bool edge_lane = lane == 0 || lane == 31;
+  const int BS = (C + 3) * FS;  // quads between row blocks
+  Q4* const F = reinterpret_cast<Q4*>(sm + l.fld) + (comp ? rb : 0) * BS + 2 * FS + lane;
+  const u64* const FU = lane > 0 ? &(F + 31)->b : rb > 0 ? &(F + 63 - BS)->b : &(F + 32)->a;
+  const float* const FD = reinterpret_cast<const float*>(
+      lane < 31 ? F + 33 : rb < RB - 1 ? F + 1 + BS : F + 32) + (lane == 31 && rb >= RB - 1 ? 3 : 0);
+  u64* const ED = reinterpret_cast<u64*>(sm + l.edge) + (rb + 1) * C * 2;
   ulonglong2* const CF = reinterpret_cast<ulonglong2*>(sm + l.col);
-  u64* const ROW = reinterpret_cast<u64*>(sm + l.row);
+  ulonglong2* const SH = reinterpret_cast<ulonglong2*>(sm + l.halo) + (comp ? rb : 0) * 256 + 2 * lane;
+  Q4* const ROW = reinterpret_cast<Q4*>(sm + l.row) + rb * 32 + lane;
+  const int NP = RB * 32;
   float* const TERM = reinterpret_cast<float*>(sm + l.term);
   float* const AMP = reinterpret_cast<float*>(sm + l.amp);
-  unsigned* const WM = reinterpret_cast<unsigned*>(sm + l.misc);       // [3][16] warp maxima
-  float* const SC = reinterpret_cast<float*>(sm + l.misc + 48 * 4);    // scales
+  unsigned* const WM = reinterpret_cast<unsigned*>(sm + l.misc);     // [3] maxima: p, vx, vz
+  float* const SC = reinterpret_cast<float*>(sm + l.misc + 16 * 4);  // scales
   unsigned* const TB = reinterpret_cast<unsigned*>(sm + l.misc + 64 * 4);
-  const int own = 32 * warp + lane;
-  const int NP = RB * 32;
+  const unsigned top = lane == 0, bottom = lane == 31;
   Poll poll{L.err, false};
   const int4 ih = S.inj.pts > 0 ? S.inj.head[b] : make_int4(0, 0, 0, 0);
   const int ipts = ih.y > 0 ? C * ih.y : 0;
@@ -386,55 +465,90 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tbase = *TB + ((unsigned)(warp & 3) << 21);  // lane 32 (warp % 4)
-  const unsigned TP = tbase + (warp >> 2) * C * 4;            // px, pz of column j: + 4 j
+  sync_cta();
+  // px, pz of column j: TP + 8 j (lane 32 (warp % 4) of the allocation)
+  const unsigned TQ = __shfl_sync(kAll, *TB, 0) + ((unsigned)(warp & 3) << 21);
+  const unsigned TP = TQ + (rb >> 2) * (C + 3) * 8 + 8;
+  const unsigned TK = TQ + group_warps(RB) / 4 * (C + 3) * 8 + (rb >> 2) * C * 4;  // kappa: TK + 4 j
   {
     const int off = kF ? 2 : 3;
     const int hi1 = g.n1e - off, hi2 = g.n2e - off;
+    const int fsrows = g.ofs == 1 ? npml + 1 : 0;
     for (int j = tid; j < C; j += blockDim.x) {
       const int c = c0 + j;
       const bool in = c < g.n2e, u = c >= 2 && c < hi2;
       const float4 q = in ? md.pcol[c] : make_float4(0.f, 0.f, 0.f, 0.f);
-      CF[2 * j] = make_ulonglong2(pk(q.x, q.x), u ? pk(q.y, q.y) : 0ull);
+      CF[2 * j] = make_ulonglong2(pk(q.x, q.x), pk(q.y, q.y));
       const float w = RHO ? 1.f : q.w;
       CF[2 * j + 1] = make_ulonglong2(pk(q.z, q.z), u ? pk(w, w) : 0ull);
     }
-    if (!aux) {
-      const bool u0 = i1 >= 2 && i1 < hi1, u1 = i1 + 1 >= 2 && i1 + 1 < hi1;
-      const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 a = i1 < g.n1e ? md.prow[i1] : z4, c = i1 + 1 < g.n1e ? md.prow[i1 + 1] : z4;
-      ROW[own] = pk(a.x, c.x);
-      ROW[NP + own] = pk(u0 ? a.y : 0.f, u1 ? c.y : 0.f);
-      ROW[2 * NP + own] = pk(a.z, c.z);
-      ROW[3 * NP + own] = pk(u0 ? (RHO ? 1.f : a.w) : 0.f, u1 ? (RHO ? 1.f : c.w) : 0.f);
-      const int fsrows = g.ofs == 1 ? npml + 1 : 0;
-      ROW[4 * NP + own] = pk(i1 < fsrows ? 0.f : 1.f, i1 + 1 < fsrows ? 0.f : 1.f);
-      for (int j = 0; j < C; ++j) {
+    if (comp) {
+      bool u[4];
+      if (cg == 0) {
+        float f[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int r = i1 + k;
+          const float4 q = r < g.n1e ? md.prow[r] : make_float4(0.f, 0.f, 0.f, 0.f);
+          f[0][k] = q.x;
+          f[1][k] = q.y;
+          f[2][k] = q.z;
+          f[3][k] = r >= 2 && r < hi1 ? (RHO ? 1.f : q.w) : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sts4(ROW + k * NP, pk4(f[k][0], f[k][1], f[k][2], f[k][3]));
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) u[k] = i1 + k >= max(2, fsrows) && i1 + k < hi1;
+      for (int j = clo; j < chi; ++j) {
         const int c = c0 + j;
-        u64 x = 0ull, z = 0ull, k = 0ull, px = 0ull, pz = 0ull;
-        if (c < g.n2e) {
+        Q4 x = kZero4, z = kZero4, k4 = kZero4, px = kZero4, pz = kZero4;
+        if (c < g.n2e && i1 < ld) {
           const size_t o = (size_t)c * ld + i1;
-          k = *reinterpret_cast<const u64*>(md.kap + o);
+          if (c >= 2 && c < hi2) {
+            // kappa (dtdx kappa where only that is used), zero where the
+            // pressure is not updated or is zeroed at the free surface: px and
+            // pz then stay zero there
+            const float4 q = *reinterpret_cast<const float4*>(md.kap + o);
+            const float s = kB ? 1.f : g.dtdx;
+            k4 = pk4(u[0] ? fmul(s, q.x) : 0.f, u[1] ? fmul(s, q.y) : 0.f,
+                     u[2] ? fmul(s, q.z) : 0.f, u[3] ? fmul(s, q.w) : 0.f);
+          }
           if (L.load) {
-            x = *reinterpret_cast<const u64*>(S.vx + o);
-            z = *reinterpret_cast<const u64*>(S.vz + o);
-            px = *reinterpret_cast<const u64*>(S.px + o);
-            pz = *reinterpret_cast<const u64*>(S.pz + o);
+            x = lds4(reinterpret_cast<const Q4*>(S.vx + o));
+            z = lds4(reinterpret_cast<const Q4*>(S.vz + o));
+            px = lds4(reinterpret_cast<const Q4*>(S.px + o));
+            pz = lds4(reinterpret_cast<const Q4*>(S.pz + o));
           }
         }
-        F[96 * j] = x;
-        F[96 * j + 32] = z;
-        F[96 * j + 64] = k;
-        tm_st4(TP + 4 * j, px, pz);
+        sts4(F + FS * j, x);
+        sts4(F + FS * j + 32, z);
+        __syncwarp();
+        tm_st(TP + 8 * j, px, pz);
+        tm_st(TK + 4 * j, k4);
+      }
+      // the neighbours' columns: zero where there is no neighbour, their vx of
+      // the state where the first step needs it
+      if (cg == 0)
+        for (int j = -2; j <= C; j = j == -1 ? C : j + 1) {
+          const int c = c0 + j;
+          Q4 x = kZero4;
+          if (L.load && c >= 0 && c < g.n2e && i1 < ld)
+            x = lds4(reinterpret_cast<const Q4*>(S.vx + (size_t)c * ld + i1));
+          sts4(F + FS * j, x);
+          sts4(F + FS * j + 32, kZero4);
+        }
+      __syncwarp();
+      if (cg == 0) {
+        tm_st(TP - 8, kZero4, kZero4);
+        tm_st(TP + 8 * C, kZero4, kZero4);
+        tm_st(TP + 8 * C + 8, kZero4, kZero4);
       }
       tm_wait_st();
     }
     for (int k = tid; k < C * 2 * (RB + 2); k += blockDim.x)
       reinterpret_cast<u64*>(sm + l.edge)[k] = 0ull;
-    if (tid < 48) WM[tid] = 0u;
+    if (tid < 3) WM[tid] = 0u;
     if (tid < 8) SC[tid] = 1.f;
     if (ipts > 0) {
       const size_t o = (size_t)b * S.inj.pts;
@@ -449,59 +563,94 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
         const int s = in ? S.inj.sta[(o + p) * S.inj.m + e] : 0xffff;
         tst[k] = (unsigned short)(s < ih.w ? s : ih.w);
       }
-      for (int k = tid; k < ipts; k += blockDim.x) tk[k] = S.inj.kap[o + k];
+      for (int k = tid; k < ipts; k += blockDim.x)  // rows above the surface: px stays zero
+        tk[k] = ih.x + k % ih.y < fsrows ? 0.f : S.inj.kap[o + k];
       for (int k = tid; k <= ih.w; k += blockDim.x)
         AMP[k] = k < ih.w ? S.amp[(size_t)(first - 1) * S.nsta + ih.z + k] : 0.f;
     }
   }
   __syncthreads();
-  if (ipts > 0 && !aux) inj_terms(sm, l, ipts, im, ncomp);
+  if (ipts > 0) inj_terms(sm, l, ipts, im);
 
   const u64 nz = L.nz;
   auto mul2 = [&](u64 x, u64 y) { return fma2(x, y, nz); };
+  auto mul4 = [&](Q4 x, Q4 y) -> Q4 { return {mul2(x.a, y.a), mul2(x.b, y.b)}; };
+  auto mul41 = [&](Q4 x, u64 y) -> Q4 { return {mul2(x.a, y), mul2(x.b, y)}; };
   // ---- per-lane constants
-  const bool r0 = i1 >= npml && i1 < npml + g.n1, r1 = i1 + 1 >= npml && i1 + 1 < npml + g.n1;
-  const bool r01 = (r0 || r1) && !aux;
-  const unsigned m0 = r0 ? 0x7fffffffu : 0u, m1 = r1 ? 0x7fffffffu : 0u;
+  unsigned rows = 0;  // bit k: row i1 + k is physical
+#pragma unroll
+  for (int k = 0; k < 4; ++k) rows |= (i1 + k >= npml && i1 + k < npml + g.n1 ? 1u : 0u) << k;
+  if (!comp) rows = 0;
+  // a warp with quads only part of which is physical masks its values
+  const bool part = __any_sync(kAll, rows != 0 && rows != 15u);
+  auto keep = [&](Q4 v, unsigned bits) -> Q4 {
+    const float4 f = up4(v);
+    return pk4(bits & 1 ? f.x : 0.f, bits & 2 ? f.y : 0.f, bits & 4 ? f.z : 0.f, bits & 8 ? f.w : 0.f);
+  };
+  // running max |x|, NaN if any value is
+  auto amax = [&](float m, Q4 v) {
+    if (part) v = keep(v, rows);
+    const float4 f = up4(v);
+    float d;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(f.x), "f"(f.y));
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(d), "f"(f.z), "f"(f.w));
+    return m;
+  };
+  auto splat = [](float v) { return pk(v, v); };
   const int jlo = max(0, npml - c0), jhi = min(C, npml + g.n2 - c0);  // physical columns [jlo, jhi)
   const unsigned phys = jhi > jlo ? (1u << jhi) - (1u << jlo) : 0u;
-  const unsigned lphys = r01 ? phys : 0u;  // of lanes with a physical row
+  const unsigned lphys = rows ? phys : 0u;  // of lanes with a physical row
   const int n1h = L.n1h;
   const size_t nih = (size_t)n1h * g.n2;
   const int hoff = i1 - g.hist_base() + n1h * (c0 - npml);  // history offset of column 0
   constexpr int kEs = FP16 ? 2 : 4;
   auto hist_at = [&](int slot, int f) {
-    return static_cast<char*>(S.hist) + (((size_t)slot * 3 + f) * nih + hoff) * kEs;
+    return static_cast<char*>(S.hist) + ((size_t)slot * 3 + f) * nih * kEs;
   };
-  const int hstep = n1h * kEs;  // bytes from one column's pair to the next
+  const int hstep = n1h * kEs;  // bytes from one column to the next
   const u64 A0 = pk(kA0, kA0), A1 = pk(kA1, kA1), DTDX = pk(g.dtdx, g.dtdx);
   const float mdt = fmul(-1.0f, g.dt);
   const u64 MDT = pk(mdt, mdt);
   const uint64_t pol = l2_evict_first();
-  // halo words: [phase][parity][cta][3][NP]
-  const size_t hcta = (size_t)3 * NP, hpar = hcta * gridDim.x;
-  ulonglong2* const hmine = L.halo + (size_t)blockIdx.x * hcta + own;
+  // halo words: [phase][parity][cta][3][NP][2]
+  const size_t hcol = (size_t)2 * NP, hcta = 3 * hcol, hpar = hcta * gridDim.x;
+  ulonglong2* const hmine = L.halo + (size_t)blockIdx.x * hcta + 2 * (32 * rb + lane);
   const bool hasl = b > 0, hasr = b + 1 < G;
-  const bool inj_on = ipts > 0 && !aux && i1 + 1 >= ih.x && i1 < ih.x + ih.y;
-  const bool inj_warp = ipts > 0 && !aux && 64 * warp + 63 >= ih.x && 64 * warp < ih.x + ih.y;
-  // rectangles kept for the gathers
-  bool rect_warp = false;
+  const bool inj_on = ipts > 0 && comp && i1 + 3 >= ih.x && i1 < ih.x + ih.y;
+  const bool inj_warp = !kB && ipts > 0 && comp && 128 * rb + 127 >= ih.x && 128 * rb < ih.x + ih.y;
+  // rectangles kept for the gathers: the CTA's columns, the lane's rows and the
+  // address of its first row and the CTA's first column at the current step
+  unsigned rcol[2] = {}, rrow[2] = {};
+  float* rptr[2] = {};
+  if (!kA && comp)
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
-    rect_warp |= !kA && S.rect[q].buf && 64 * warp + 63 >= S.rect[q].r0 && 64 * warp < S.rect[q].r1;
-  const bool extra = !kA && !aux && (rect_warp || S.wf != nullptr);  // warp-uniform
+    for (int q = 0; q < 2; ++q) {
+      const ResidentRect& R = S.rect[q];
+      if (!R.buf || 128 * rb + 127 < R.r0 || 128 * rb >= R.r1) continue;
+      const int a = max(R.c0 - c0, 0), e = min(R.c1 - c0, C);
+      rcol[q] = e > a ? (1u << e) - (1u << a) : 0u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) rrow[q] |= (i1 + k >= R.r0 && i1 + k < R.r1 ? 1u : 0u) << k;
+      rptr[q] = R.buf + (ptrdiff_t)(i1 - R.r0) * R.ld + (c0 - R.c0);
+    }
+  // warps with more to do per column than the update (warp-uniform)
+  const bool extra = !kA && comp && ((rcol[0] | rcol[1]) != 0 || S.wf != nullptr);
   // free-surface copy vz(npml - 1) = vz(npml)
-  const bool fs_warp = g.ofs == 1 && (npml - 1) / 64 == warp;
-  const int slo = L.slo, shi1 = g.n1 - L.slo;
+  const bool fs_warp = g.ofs == 1 && (npml - 1) / 128 == rb;
+  const int fsk = npml - 1 - i1;  // 0 .. 3 in the lane that owns row npml - 1
+  const int slo = L.slo;
   const int sjlo = max(0, npml + slo - c0), sjhi = min(C, npml + g.n2 - slo - c0);
   const unsigned srcs = sjhi > sjlo ? (1u << sjhi) - (1u << sjlo) : 0u;  // source columns
-  const unsigned lsrc = r01 ? srcs : 0u;
-  const bool s0 = r0 && i1 - npml >= slo && i1 - npml < shi1;
-  const bool s1 = r1 && i1 + 1 - npml >= slo && i1 + 1 - npml < shi1;
-  HT hq[U] = {}, hx[U] = {}, hz[U] = {};  // stage B: history pairs read ahead
+  const unsigned lsrc = rows ? srcs : 0u;
+  unsigned srows = 0;  // rows of the pressure source
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    srows |= (i1 + k >= npml + slo && i1 + k < npml + g.n1 - slo ? 1u : 0u) << k;
+  const bool spart = kB && __any_sync(kAll, (srows & rows) != rows);
+  HT hq[HR] = {}, hx[HR] = {}, hz[HR] = {};  // stage B: history quads read ahead
   auto slot_b = [&](int it) { return S.nt - it - L.hist_step0; };  // the time-reversed step's
   auto ldh = [&](const char* base, int j, unsigned mask) -> HT {
-    return HP::load(base + (ptrdiff_t)j * hstep, mask >> j & 1u);
+    return HQ::load(base + (ptrdiff_t)(hoff + j * n1h) * kEs, mask >> j & 1u);
   };
   // stage B: scales of one step (extra warp), and the L2 prefetch of its history
   auto scales_b = [&](int it) {
@@ -520,213 +669,195 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
                       (((size_t)slot_b(it) * 3 + lane) * nih + (size_t)(c0 + jlo - npml) * n1h) * kEs,
                   (unsigned)((jhi - jlo) * n1h * kEs));
   };
+  const bool ledge = comp && clo == 0, redge = comp && chi == C;
+  // the warp's first columns of the pressure and velocity half steps
+  const int pj0 = chi > 2 ? max(clo, 2) : clo, vj0 = ledge && chi > 1 ? 1 : clo;
   if (kB) {
     if (aux) {
       scales_b(first);
       prefetch_b(first + 1);
-    } else {
+    } else if (comp) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) hq[u] = ldh(hist_at(slot_b(first), 0), 2 + u, lsrc);
+      for (int u = 0; u < HR; ++u) hq[u] = ldh(hist_at(slot_b(first), 0), pj0 + u, lsrc);
     }
   }
-  const u64 fsm = aux ? 0ull : ROW[4 * NP + own];
-  __syncthreads();
+  sync_cta();
 
   for (int it = first; it <= last; ++it) {
     const unsigned tag = L.tag0 + (unsigned)it;
     // =============== pressure half step ===============
-    if (!aux) {
-      const u64 d1a = ROW[own], d1a1 = ROW[NP + own];
-      const float inv = kA && FP16 ? SC[0] : 1.f;
-      const u64 INV = pk(r0 ? inv : 0.f, r1 ? inv : 0.f);
-      const unsigned putm = kA && it > first ? 0xffffffffu : 0u;
+    if (comp) {
+      const Q4 d1a = lds4(ROW), d1a1 = lds4(ROW + NP);
+      const u64 INV = splat(kA && FP16 ? SC[0] : 1.f), SCP = splat(kB ? SC[(it & 1) * 3] : 1.f);
+      const unsigned put = kA && it > first && rows ? 1u : 0u;
       char* const hp = hist_at(kA ? max(it - 2, 0) : slot_b(it), 0);
-      const float scp = kB ? SC[(it & 1) * 3] : 1.f;
-      const u64 SCP = pk(s0 ? scp : 0.f, s1 ? scp : 0.f);
-      unsigned lmax = 0;
+      float lmax = 0.f;
       ulonglong2* const hout = hmine + (size_t)(it & 1) * hpar;  // phase 0: p words
-      // One column j, its arrays at f, fu, fd, cf, ed, tp, hb: qm2 .. qp1 are
-      // vx of columns j-2 .. j+1, h the history pair, `on` whether this lane has
-      // physical points of the column.
-      auto column = [&](int j, u64* f, const u64* fu, const u64* fd, const ulonglong2* cfp, u64* ed,
-                        unsigned tp, char* hb, unsigned on, u64 qm2, u64 qm1, u64 q0, u64 qp1,
-                        HT h) {
-        unsigned t4[4];
-        tm_ld4(tp, t4);
-        const float2 z = up(f[32]), zm = up(*fu);
-        const float zp2 = *reinterpret_cast<const float*>(fd);
-        const u64 kap = f[64];
-        const ulonglong2 cf = *cfp;
-        const u64 der2 = add2(mul2(A0, sub2(q0, qm1)), mul2(A1, sub2(qp1, qm2)));
-        const u64 der1 = add2(mul2(A0, pk(fsub(z.x, zm.y), fsub(z.y, z.x))),
-                              mul2(A1, pk(fsub(z.y, zm.x), fsub(zp2, zm.y))));
-        const u64 kd = mul2(DTDX, kap);
-        const u64 bx = mul2(mul2(kd, cf.y), der2), bz = mul2(mul2(kd, d1a1), der1);
-        tm_wait(t4);
-        u64 px = pku(t4[0], t4[1]), pz = pku(t4[2], t4[3]);
-        if (kA)  // history of the previous step's pressure
-          HP::put(hb, mul2(mul2(fsm, add2(px, pz)), INV), pol, on & putm);
-        const u64 ax = mul2(cf.x, px), az = mul2(d1a, pz);
-        px = kA ? sub2(ax, bx) : add2(ax, bx);
-        pz = kA ? sub2(az, bz) : add2(az, bz);
-        if (!kB && inj_warp) {
-          if (inj_on) {
-            const float2* t =
-                reinterpret_cast<const float2*>(TERM + (size_t)(j * ih.y + (i1 - ih.x)) * im);
-            float2 v = up(px);
-            for (int k = 0; k < im / 2; ++k) {
-              const float2 t0 = t[k], t1 = t[im / 2 + k];
-              v.x = kA ? fsub(fsub(v.x, t0.x), t0.y) : fadd(fadd(v.x, t0.x), t0.y);
-              v.y = kA ? fsub(fsub(v.y, t1.x), t1.y) : fadd(fadd(v.y, t1.x), t1.y);
+      const ulonglong2* const hin = hmine + (size_t)(2 + ((it - 1) & 1)) * hpar;  // vx words
+      // The warp's columns in order, those of the left edge (0 and 1) last: the
+      // neighbours' words are fetched two columns before the last one between
+      // the edges and put into columns C, -2 and -1 when they are needed.
+      const int jx = chi > 2 ? max(pj0, min(chi, C - 1) - 2) : 31;
+      const bool rhalo = hasr && redge && it > first, lhalo = hasl && clo < 2 && it > first;
+      const unsigned events = (1u << jx) | (rhalo ? 1u << (C - 1) : 0u);
+      const unsigned outs = (hasr ? 1u << (C - 1) : 0u) | (hasl ? 3u : 0u);
+      HT he[HR] = {};  // histories of columns 0 and 1
+      auto fetch = [&]() {
+        if (rhalo) halo_fetch<1>(SH + 128, hin + hcta + 2 * hcol, hcol);
+        if (lhalo) halo_fetch<2>(SH, hin - hcta, hcol);
+        if (kB && ledge) {
+          he[0] = ldh(hp, 0, lsrc);
+          he[1] = ldh(hp, 1, lsrc);
+        }
+      };
+      auto put_left = [&]() {
+        if (!lhalo) return;
+        Q4 h[2];
+        halo_get(SH, hin - hcta, hcol, tag - 1, poll, h);
+        sts4(F - 2 * FS, h[0]);
+        sts4(F - FS, h[1]);
+      };
+      auto put_right = [&]() {
+        Q4 r[1];
+        halo_get(SH + 128, hin + hcta + 2 * hcol, hcol, tag - 1, poll, r);
+        sts4(F + FS * C, r[0]);
+      };
+      // Columns [j, je): four to an iteration, so that the window's registers
+      // rotate without copies.  Arrays at column j, masks shifted by j.
+      auto columns = [&](int j, int je) {
+        Q4* f = F + FS * j;
+        const u64* fu = FU + 2 * FS * j;
+        const float* fd = FD + 4 * FS * j;
+        const ulonglong2* cf = CF + 2 * j;
+        u64* ed = ED + 2 * j;
+        unsigned tp = TP + 8 * j, tk = TK + 4 * j, ho = (unsigned)((hoff + j * n1h) * kEs);
+        unsigned ev = events >> j, ot = outs >> j, ph = phys >> j, src = lsrc >> j;
+        int n = je - j;
+        Q4 w0 = lds4(f - 2 * FS), w1 = lds4(f - FS), w2 = lds4(f), w3;
+        auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
+          if (ev & (1u << k)) {
+            if (j + k == jx) fetch();
+            if (rhalo && j + k == C - 1) put_right();
+          }
+          w3 = lds4(f + FS * (k + 1));
+          const float4 z = up4(lds4(f + FS * k + 32));
+          const float2 zm = up(fu[2 * FS * k]);
+          const float zp = fd[4 * FS * k];
+          const ulonglong2 c2 = cf[2 * k];
+          Q4 px, pz, kap;
+          tm_ld(tp + 8 * k, tk + 4 * k, px, pz, kap);
+          const Q4 der2 = add4(mul41(sub4(w2, w1), A0), mul41(sub4(w3, w0), A1));
+          const Q4 der1 = add4(mul41(pk4(fsub(z.x, zm.y), fsub(z.y, z.x), fsub(z.z, z.y), fsub(z.w, z.z)), A0),
+                               mul41(pk4(fsub(z.y, zm.x), fsub(z.z, zm.y), fsub(z.w, z.x), fsub(zp, z.y)), A1));
+          if (kA && (ph & (1u << k))) {  // history of the previous step's pressure
+            Q4 v = mul41(add4(px, pz), INV);
+            if (part) v = keep(v, rows);
+            HQ::put(hp + (ho + k * hstep), v, pol, put);
+          }
+          const Q4 kd = kB ? mul41(kap, DTDX) : kap;
+          const Q4 bx = mul4(mul41(kd, c2.y), der2), bz = mul4(mul4(kd, d1a1), der1);
+          const Q4 ax = mul41(px, c2.x), az = mul4(d1a, pz);
+          px = kA ? sub4(ax, bx) : add4(ax, bx);
+          pz = kA ? sub4(az, bz) : add4(az, bz);
+          if (inj_warp) {
+            if (inj_on) {  // the lane's four rows are rows of the table
+              float4 v = up4(px);
+              const float2* t =
+                  reinterpret_cast<const float2*>(TERM + ((j + k) * ih.y + (i1 - ih.x)) * im);
+              const int mh = im >> 1;
+              for (int q = 0; q < mh; ++q) {
+                const float2 a = t[q], e = t[mh + q], c = t[2 * mh + q], d = t[3 * mh + q];
+                v.x = kA ? fsub(fsub(v.x, a.x), a.y) : fadd(fadd(v.x, a.x), a.y);
+                v.y = kA ? fsub(fsub(v.y, e.x), e.y) : fadd(fadd(v.y, e.x), e.y);
+                v.z = kA ? fsub(fsub(v.z, c.x), c.y) : fadd(fadd(v.z, c.x), c.y);
+                v.w = kA ? fsub(fsub(v.w, d.x), d.y) : fadd(fadd(v.w, d.x), d.y);
+              }
+              px = pk4(v.x, v.y, v.z, v.w);
             }
-            px = pk(v.x, v.y);
+            __syncwarp();
           }
-          __syncwarp();
+          if (kB) {  // points outside the physical range read 0
+            Q4 v = mul41(HQ::get(hq[k % HR]), SCP);
+            if (spart) v = keep(v, srows);
+            px = add4(px, mul4(mul41(v, MDT), kap));
+            hq[k % HR] = HQ::load(hp + (ho + (k + HR) * hstep), src & (1u << (k + HR)));
+          }
+          tm_st(tp + 8 * k, px, pz);
+          const Q4 p = add4(px, pz);
+          sts_if(ed + 2 * k, p.a, top);
+          sts_if(ed + 2 * k + 1, p.b, bottom);
+          if (kA && (ph & (1u << k))) lmax = amax(lmax, p);
+          if (extra) {
+            // pressure rows of the gather rectangles, and the wavefield output
+            const float4 v = up4(p);
+            if (rcol[0] >> (j + k) & 1u) stg_rows(rptr[0] + j + k, S.rect[0].ld, v, rrow[0]);
+            if (rcol[1] >> (j + k) & 1u) stg_rows(rptr[1] + j + k, S.rect[1].ld, v, rrow[1]);
+            if (S.wf && (ph & (1u << k))) {
+              float* w = S.wf + (size_t)(it - 1) * g.int_elems() + (size_t)g.n1 * (c0 + j + k - npml) + (i1 - npml);
+              const bool acc = S.wf_acc != 0;
+              if (rows & 1u) w[0] = acc ? fadd(w[0], v.x) : v.x;
+              if (rows & 2u) w[1] = acc ? fadd(w[1], v.y) : v.y;
+              if (rows & 4u) w[2] = acc ? fadd(w[2], v.z) : v.z;
+              if (rows & 8u) w[3] = acc ? fadd(w[3], v.w) : v.w;
+              __syncwarp();
+            }
+          }
+          // to the neighbours: the last column to the right, 0 and 1 to the left
+          if (ot & (1u << k)) ll_store(hout + (j + k < 2 ? 1 + j + k : 0) * hcol, p, tag);
+        };
+        for (;;) {
+          column(0, w0, w1, w2, w3);
+          if (n == 1) break;
+          column(1, w1, w2, w3, w0);
+          if (n == 2) break;
+          column(2, w2, w3, w0, w1);
+          if (n == 3) break;
+          column(3, w3, w0, w1, w2);
+          if (n == 4) break;
+          n -= 4;
+          j += 4;
+          f += 4 * FS;
+          fu += 8 * FS;
+          fd += 16 * FS;
+          cf += 8;
+          ed += 8;
+          tp += 32;
+          tk += 16;
+          ho += 4 * hstep;
+          ev >>= 4;
+          ot >>= 4;
+          ph >>= 4;
+          src >>= 4;
         }
-        // lanes outside the source range have a zero scale or read no history
-        if (kB) px = add2(px, mul2(mul2(MDT, mul2(HP::get(h), SCP)), kap));
-        tm_st4(tp, px, pz);
-        const u64 p = mul2(fsm, add2(px, pz));
-        sts_if(ed, p, edge_lane);
-        if (kA) {
-          const float2 pv = up(p);
-          if (on) lmax = max(lmax, max(__float_as_uint(pv.x) & m0, __float_as_uint(pv.y) & m1));
-        }
-        return p;
       };
-      auto column_at = [&](int j, u64 qm2, u64 qm1, u64 q0, u64 qp1, HT h) {
-        return column(j, F + 96 * j, FU + 96 * j, FD + 96 * j, CF + 2 * j, EDL + 2 * j, TP + 4 * j,
-                      hp + (ptrdiff_t)j * hstep, lphys >> j & 1u, qm2, qm1, q0, qp1, h);
-      };
-      // columns 2 .. C-2, U at a time, then one by one
-      u64 q[U + 3];
-      q[0] = F[0];
-      q[1] = F[96];
-      q[2] = F[192];
-      {
-        u64* f = F + 192;
-        const u64 *fu = FU + 192, *fd = FD + 192;
-        const ulonglong2* cf = CF + 4;
-        u64* ed = EDL + 4;
-        unsigned tp = TP + 8, on = (kB ? lsrc : lphys) >> 2;
-        char* hb = hp + 2 * (ptrdiff_t)hstep;
-        int j = 2;
-        for (; j + U <= C - 1; j += U) {
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            q[u + 3] = f[96 * (u + 1)];
-            column(j + u, f + 96 * u, fu + 96 * u, fd + 96 * u, cf + 2 * u, ed + 2 * u, tp + 4 * u, hb,
-                   on & (1u << u), q[u], q[u + 1], q[u + 2], q[u + 3], hq[u]);
-            if (kA) hb += hstep;
-            // source columns beyond C - 1 have no bit
-            if (kB) hq[u] = HP::load(hb + (ptrdiff_t)(u + U) * hstep, on & (1u << (u + U)));
-          }
-          q[0] = q[U];
-          q[1] = q[U + 1];
-          q[2] = q[U + 2];
-          f += 96 * U;
-          fu += 96 * U;
-          fd += 96 * U;
-          cf += 2 * U;
-          ed += 2 * U;
-          tp += 4 * U;
-          on >>= U;
-          if (kB) hb += (ptrdiff_t)U * hstep;
+      for (int j = pj0, je = chi;;) {
+        if (j < 2) {
+          if (je <= 2) fetch();
+          put_left();
         }
-#pragma unroll 1
-        for (; j < C - 1; ++j) {
-          const u64 qn = f[96];
-          column(j, f, fu, fd, cf, ed, tp, hb, on & 1u, q[0], q[1], q[2], qn, hq[0]);
-          q[0] = q[1];
-          q[1] = q[2];
-          q[2] = qn;
-          hq[0] = hq[1];
-          hq[1] = hq[2];
-          f += 96;
-          fu += 96;
-          fd += 96;
-          cf += 2;
-          ed += 2;
-          tp += 4;
-          on >>= 1;
-          hb += hstep;
+        columns(j, je);
+        if (clo > 0 || je <= 2) break;
+        j = 0;  // the left edge's columns
+        je = 2;
+        if (kB) {
+          hq[0] = he[0];
+          hq[1] = he[1];
         }
       }
-      // the last column, with the right neighbour's first
-      HT he[3] = {};
-      if (kB) {
-        he[0] = ldh(hp, C - 1, lsrc);
-        he[1] = ldh(hp, 0, lsrc);
-        he[2] = ldh(hp, 1, lsrc);
-      }
-      u64 qd = 0ull;
-      if (hasr) {
-        if (it == first) {
-          const int c = c0 + C;
-          if (L.load && c < g.n2e) qd = *reinterpret_cast<const u64*>(S.vx + (size_t)c * ld + i1);
-        } else {
-          qd = ll_wait1(hmine + (size_t)(2 + ((it - 1) & 1)) * hpar + hcta + 2 * NP, tag - 1, poll);
-        }
-      }
-      const u64 pe = column_at(C - 1, q[0], q[1], q[2], qd, he[0]);
-      if (hasr) ll_store(hout, pe, tag);
-      // columns 0 and 1, with the left neighbour's last two
-      u64 ha = 0ull, hb = 0ull;
-      if (hasl) {
-        if (it == first) {
-          if (L.load) {
-            ha = *reinterpret_cast<const u64*>(S.vx + (size_t)(c0 - 2) * ld + i1);
-            hb = *reinterpret_cast<const u64*>(S.vx + (size_t)(c0 - 1) * ld + i1);
-          }
-        } else {
-          const ulonglong2* h = hmine + (size_t)(2 + ((it - 1) & 1)) * hpar - hcta;
-          ll_wait2(h, h + NP, tag - 1, poll, ha, hb);
-        }
-      }
-      const u64 qa = F[0], qb = F[96], qc = F[192];
-      const u64 p0 = column_at(0, ha, hb, qa, qb, he[1]);
-      if (hasl) ll_store(hout + NP, p0, tag);
-      const u64 p1 = column_at(1, hb, qa, qb, qc, he[2]);
-      if (hasl) ll_store(hout + 2 * NP, p1, tag);
       tm_wait_st();
       if (kA) {
-        lmax = __reduce_max_sync(kAll, lmax);
-        if (lane == 0) WM[warp] = lmax;
+        const unsigned m = __reduce_max_sync(kAll, rows ? __float_as_uint(lmax) & 0x7fffffffu : 0u);
+        if (lane == 0) atomicMax(&WM[0], m);
       }
       if (kB) {  // velocity histories of the first columns of the next half step
         const char *hbx = hist_at(slot_b(it), 1), *hbz = hist_at(slot_b(it), 2);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          hx[u] = ldh(hbx, 1 + u, lphys);
-          hz[u] = ldh(hbz, 1 + u, lphys);
+        for (int u = 0; u < HR; ++u) {
+          hx[u] = ldh(hbx, vj0 + u, lphys);
+          hz[u] = ldh(hbz, vj0 + u, lphys);
         }
       }
-      if (extra) {
-        // pressure rows of the gather rectangles, and the wavefield output
-        for (int j = 0; j < C; ++j) {
-          unsigned t4[4];
-          tm_ld4(TP + 4 * j, t4);
-          tm_wait(t4);
-          const float2 pv = up(mul2(fsm, add2(pku(t4[0], t4[1]), pku(t4[2], t4[3]))));
-          const int c = c0 + j;
-#pragma unroll
-          for (int q2 = 0; q2 < 2; ++q2) {
-            const ResidentRect& R = S.rect[q2];
-            if (R.buf && c >= R.c0 && c < R.c1) {
-              float* o2 = R.buf + (size_t)(it - first) * R.step + (ptrdiff_t)(i1 - R.r0) * R.ld + (c - R.c0);
-              if (i1 >= R.r0 && i1 < R.r1) o2[0] = pv.x;
-              if (i1 + 1 >= R.r0 && i1 + 1 < R.r1) o2[R.ld] = pv.y;
-            }
-          }
-          if (S.wf && (phys >> j & 1u)) {
-            float* w = S.wf + (size_t)(it - 1) * g.int_elems() + (size_t)g.n1 * (c - npml) + (i1 - npml);
-            if (r0) w[0] = S.wf_acc ? fadd(w[0], pv.x) : pv.x;
-            if (r1) w[1] = S.wf_acc ? fadd(w[1], pv.y) : pv.y;
-          }
-          __syncwarp();
-        }
-      }
-    } else {
+    } else if (aux) {
       if (!kB && ipts > 0 && it < last)  // amplitudes of the next step
         for (int k = lane; k < ih.w; k += 32) AMP[k] = S.amp[(size_t)it * S.nsta + ih.z + k];
       if (kA && it > first) {            // velocity maxima of the previous step
@@ -747,192 +878,200 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
       }
       if (kB) prefetch_b(it + 2);
     }
-    __syncthreads();
+    if (extra) {
+      rptr[0] += S.rect[0].step;
+      rptr[1] += S.rect[1].step;
+    }
+    sync_cta();
     // =============== velocity half step ===============
-    if (!aux) {
-      if (!kB && ipts > 0 && it < last) inj_terms(sm, l, ipts, im, ncomp);
-      const u64 d1b = ROW[2 * NP + own], bw1 = ROW[3 * NP + own];
-      const float ix = kA && FP16 ? SC[1] : 1.f, iz = kA && FP16 ? SC[2] : 1.f;
-      const u64 INVX = pk(r0 ? ix : 0.f, r1 ? ix : 0.f), INVZ = pk(r0 ? iz : 0.f, r1 ? iz : 0.f);
-      const unsigned putm = kA && it > first ? 0xffffffffu : 0u;
+    if (!kB && ipts > 0 && it < last) inj_terms(sm, l, ipts, im);
+    if (comp) {
+      const Q4 d1b = lds4(ROW + 2 * NP), bw1 = lds4(ROW + 3 * NP);
+      const u64 INVX = splat(kA && FP16 ? SC[1] : 1.f), INVZ = splat(kA && FP16 ? SC[2] : 1.f);
+      const unsigned put = kA && it > first && rows ? 1u : 0u;
       char* const hpx = hist_at(kA ? max(it - 2, 0) : slot_b(it), 1);
       char* const hpz = hist_at(kA ? max(it - 2, 0) : slot_b(it), 2);
-      const float sx = kB ? SC[(it & 1) * 3 + 1] : 1.f, sz = kB ? SC[(it & 1) * 3 + 2] : 1.f;
-      const u64 SCX = pk(r0 ? sx : 0.f, r1 ? sx : 0.f), SCZ = pk(r0 ? sz : 0.f, r1 ? sz : 0.f);
-      unsigned lmx = 0, lmz = 0;
+      const u64 SCX = splat(kB ? SC[(it & 1) * 3 + 1] : 1.f), SCZ = splat(kB ? SC[(it & 1) * 3 + 2] : 1.f);
+      float lmx = 0.f, lmz = 0.f;
       ulonglong2* const hout = hmine + (size_t)(2 + (it & 1)) * hpar;  // phase 1: vx words
-      auto pcol = [&](unsigned (&t4)[4]) { return mul2(fsm, add2(pku(t4[0], t4[1]), pku(t4[2], t4[3]))); };
-      auto pload = [&](int j) {
-        unsigned t4[4];
-        tm_ld4(TP + 4 * j, t4);
-        tm_wait(t4);
-        return pcol(t4);
+      const ulonglong2* const hin = hmine + (size_t)(it & 1) * hpar;   // p words
+      auto pload = [&](int jj) {
+        Q4 x, z;
+        tm_ld(TP + 8 * jj, x, z);
+        return add4(x, z);
       };
-      // One column j, its arrays at f, cf, ed, hbx, hbz: pm .. p2 are p of
-      // columns j-1 .. j+2 (p2 read from the tensor memory here when tp != 0).
-      auto column = [&](int j, u64* f, const ulonglong2* cfp, const u64* ed, unsigned tp, char* hbx,
-                        char* hbz, unsigned on, u64 pm, u64 p0, u64 p1, u64& p2, HT hvx, HT hvz) {
-        unsigned t4[4];
-        if (tp) tm_ld4(tp, t4);
-        const float2 p = up(p0);
-        float pm1 = __shfl_up_sync(kAll, p.y, 1);
-        float ppx = __shfl_down_sync(kAll, p.x, 1), ppy = __shfl_down_sync(kAll, p.y, 1);
-        // the neighbouring warps' pairs: last of the warp above, first of the warp below
-        lds_if(pm1, reinterpret_cast<const float*>(ed - 2 * C + 1) + 1, lane == 0);
-        lds_if(ppx, ppy, reinterpret_cast<const float*>(ed + 2 * C), lane == 31);
-        u64 vx = f[0], vz = f[32];
-        const ulonglong2 cf = *cfp;
-        const u64 der1 = add2(mul2(A0, pk(fsub(p.y, p.x), fsub(ppx, p.y))),
-                              mul2(A1, pk(fsub(ppx, pm1), fsub(ppy, p.x))));
-        if (kA) HP::put2(hbx, mul2(vx, INVX), hbz, mul2(vz, INVZ), pol, on & putm);
-        u64 w2 = cf.y, w1 = bw1;
-        u64 bu = 0ull;
-        if (RHO) {
-          const size_t k = (size_t)min(c0 + j, g.n2e - 1) * ld + i1;
-          w2 = mul2(w2, __ldg(reinterpret_cast<const u64*>(md.rbw2 + k)));
-          w1 = mul2(w1, __ldg(reinterpret_cast<const u64*>(md.rbw1 + k)));
-          if (kB) bu = __ldg(reinterpret_cast<const u64*>(md.rbue + k));
+      // The warp's columns in order, column 0 last; the neighbours' words go into
+      // the tensor memory's columns C, C + 1 and -1.
+      const int jx = vj0 > 0 && vj0 < C - 1 ? max(vj0, min(chi, C - 2) - 2) : 31;
+      const bool rhalo = hasr && chi > C - 2, lhalo = hasl && ledge;
+      const unsigned events = (1u << jx) | (rhalo && clo <= C - 2 ? 1u << (C - 2) : 0u);
+      const unsigned outs = (hasr ? 3u << (C - 2) : 0u) | (hasl ? 1u : 0u);
+      HT ex = {}, ez = {};  // histories of column 0
+      auto fetch = [&]() {
+        if (rhalo) halo_fetch<2>(SH + 128, hin + hcta + hcol, hcol);
+        if (lhalo) halo_fetch<1>(SH, hin - hcta, hcol);
+        if (kB && ledge) {
+          ex = ldh(hpx, 0, lphys);
+          ez = ldh(hpz, 0, lphys);
         }
-        const u64 az = mul2(d1b, vz), bz = mul2(w1, der1);
-        vz = kA ? sub2(az, bz) : add2(az, bz);
-        if (tp) {
-          tm_wait(t4);
-          p2 = pcol(t4);
-        }
-        const u64 der2 = add2(mul2(A0, sub2(p1, p0)), mul2(A1, sub2(p2, pm)));
-        const u64 ax = mul2(cf.x, vx), bx = mul2(w2, der2);
-        vx = kA ? sub2(ax, bx) : add2(ax, bx);
-        if (kB) {  // outside the physical range: the term is 0 (history read as 0)
-          u64 tx = mul2(MDT, mul2(HP::get(hvx), SCX)), tz = mul2(MDT, mul2(HP::get(hvz), SCZ));
+      };
+      auto put_right = [&]() {
+        Q4 r[2];
+        halo_get(SH + 128, hin + hcta + hcol, hcol, tag, poll, r);
+        tm_st(TP + 8 * C, r[0], kZero4);
+        tm_st(TP + 8 * C + 8, r[1], kZero4);
+        tm_wait_st();
+      };
+      auto put_left = [&]() {
+        if (!lhalo) return;
+        Q4 h[1];
+        halo_get(SH, hin - hcta, hcol, tag, poll, h);
+        tm_st(TP - 8, h[0], kZero4);
+        tm_wait_st();
+      };
+      // Columns [j, je), as in the pressure half step.
+      auto columns = [&](int j, int je) {
+        Q4* f = F + FS * j;
+        const ulonglong2* cf = CF + 2 * j + 1;
+        const u64* ed = ED + 2 * j;
+        unsigned tp = TP + 8 * (j + 2), ho = (unsigned)((hoff + j * n1h) * kEs);
+        unsigned ev = events >> j, ot = outs >> j, ph = phys >> j, src = lphys >> j;
+        int n = je - j;
+        Q4 w0 = pload(j - 1), w1 = pload(j), w2 = pload(j + 1), w3;
+        auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
+          if (ev & (1u << k)) {
+            if (j + k == jx) fetch();
+            if (rhalo && j + k == C - 2) put_right();
+          }
+          const float4 p = up4(w1);
+          float pm1 = __shfl_up_sync(kAll, p.w, 1);
+          float n0 = __shfl_down_sync(kAll, p.x, 1), n1 = __shfl_down_sync(kAll, p.y, 1);
+          // the neighbouring blocks' pairs: last of the one above, first of the one below
+          lds_if(pm1, reinterpret_cast<const float*>(ed + 2 * k + 1 - 2 * C) + 1, top);
+          lds_if(n0, n1, reinterpret_cast<const float*>(ed + 2 * k + 2 * C), bottom);
+          Q4 vx = lds4(f + FS * k), vz = lds4(f + FS * k + 32), qx, qz;
+          const ulonglong2 c2 = cf[2 * k];
+          tm_ld(tp + 8 * k, qx, qz);
+          w3 = add4(qx, qz);
+          Q4 k2{c2.y, c2.y}, k1 = bw1, bu = kZero4;
           if (RHO) {
-            tx = mul2(tx, bu);
-            tz = mul2(tz, bu);
-          }
-          vx = add2(vx, tx);
-          vz = add2(vz, tz);
-        }
-        if (fs_warp) {
-          float2 v = up(vz);
-          const float below = __shfl_down_sync(kAll, v.x, 1);
-          if (i1 == npml - 1) v.x = v.y;
-          if (i1 + 1 == npml - 1) v.y = below;
-          vz = pk(v.x, v.y);
-        }
-        f[0] = vx;
-        f[32] = vz;
-        if (kA) {
-          const float2 x = up(vx), z = up(vz);
-          if (on) {
-            lmx = max(lmx, max(__float_as_uint(x.x) & m0, __float_as_uint(x.y) & m1));
-            lmz = max(lmz, max(__float_as_uint(z.x) & m0, __float_as_uint(z.y) & m1));
-          }
-        }
-        return vx;
-      };
-      auto column_at = [&](int j, u64 pm, u64 p0, u64 p1, u64 p2, HT hvx, HT hvz) {
-        return column(j, F + 96 * j, CF + 2 * j + 1, ED + 2 * j, 0u, hpx + (ptrdiff_t)j * hstep,
-                      hpz + (ptrdiff_t)j * hstep, lphys >> j & 1u, pm, p0, p1, p2, hvx, hvz);
-      };
-      const u64 P0 = pload(0), P1 = pload(1), P2 = pload(2);
-      // columns 1 .. C-3, U at a time, then one by one
-      u64 q[U + 3];
-      q[0] = P0;
-      q[1] = P1;
-      q[2] = P2;
-      {
-        u64* f = F + 96;
-        const ulonglong2* cf = CF + 3;
-        const u64* ed = ED + 2;
-        unsigned tp = TP + 12, on = lphys >> 1;
-        char *hbx = hpx + hstep, *hbz = hpz + hstep;
-        int j = 1;
-        for (; j + U <= C - 2; j += U) {
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            column(j + u, f + 96 * u, cf + 2 * u, ed + 2 * u, tp + 4 * u, hbx, hbz, on & (1u << u),
-                   q[u], q[u + 1], q[u + 2], q[u + 3], hx[u], hz[u]);
-            if (kA) {
-              hbx += hstep;
-              hbz += hstep;
-            }
+            const size_t o = (size_t)min(c0 + j + k, g.n2e - 1) * ld + min(i1, ld - 4);
+            const ulonglong2 r2 = __ldg(reinterpret_cast<const ulonglong2*>(md.rbw2 + o));
+            const ulonglong2 r1 = __ldg(reinterpret_cast<const ulonglong2*>(md.rbw1 + o));
+            k2 = mul4(k2, Q4{r2.x, r2.y});
+            k1 = mul4(k1, Q4{r1.x, r1.y});
             if (kB) {
-              hx[u] = HP::load(hbx + (ptrdiff_t)(u + U) * hstep, on & (1u << (u + U)));
-              hz[u] = HP::load(hbz + (ptrdiff_t)(u + U) * hstep, on & (1u << (u + U)));
+              const ulonglong2 r = __ldg(reinterpret_cast<const ulonglong2*>(md.rbue + o));
+              bu = {r.x, r.y};
             }
           }
-          q[0] = q[U];
-          q[1] = q[U + 1];
-          q[2] = q[U + 2];
-          f += 96 * U;
-          cf += 2 * U;
-          ed += 2 * U;
-          tp += 4 * U;
-          on >>= U;
-          if (kB) {
-            hbx += (ptrdiff_t)U * hstep;
-            hbz += (ptrdiff_t)U * hstep;
+          const Q4 der1 = add4(mul41(pk4(fsub(p.y, p.x), fsub(p.z, p.y), fsub(p.w, p.z), fsub(n0, p.w)), A0),
+                               mul41(pk4(fsub(p.z, pm1), fsub(p.w, p.x), fsub(n0, p.y), fsub(n1, p.z)), A1));
+          if (kA && (ph & (1u << k))) {
+            Q4 x = mul41(vx, INVX), z = mul41(vz, INVZ);
+            if (part) {
+              x = keep(x, rows);
+              z = keep(z, rows);
+            }
+            HQ::put(hpx + (ho + k * hstep), x, pol, put);
+            HQ::put(hpz + (ho + k * hstep), z, pol, put);
           }
+          const Q4 az = mul4(d1b, vz), bz = mul4(k1, der1);
+          vz = kA ? sub4(az, bz) : add4(az, bz);
+          const Q4 der2 = add4(mul41(sub4(w2, w1), A0), mul41(sub4(w3, w0), A1));
+          const Q4 ax = mul41(vx, c2.x), bx = mul4(k2, der2);
+          vx = kA ? sub4(ax, bx) : add4(ax, bx);
+          if (kB) {  // outside the physical range: the term is 0 (history read as 0)
+            Q4 tx = mul41(mul41(HQ::get(hx[k % HR]), SCX), MDT), tz = mul41(mul41(HQ::get(hz[k % HR]), SCZ), MDT);
+            if (RHO) {
+              tx = mul4(tx, bu);
+              tz = mul4(tz, bu);
+            }
+            vx = add4(vx, tx);
+            vz = add4(vz, tz);
+            const unsigned on = src & (1u << (k + HR));
+            hx[k % HR] = HQ::load(hpx + (ho + (k + HR) * hstep), on);
+            hz[k % HR] = HQ::load(hpz + (ho + (k + HR) * hstep), on);
+          }
+          if (fs_warp) {
+            float4 v = up4(vz);
+            const float below = __shfl_down_sync(kAll, v.x, 1);
+            if (fsk == 0) v.x = v.y;
+            if (fsk == 1) v.y = v.z;
+            if (fsk == 2) v.z = v.w;
+            if (fsk == 3) v.w = below;
+            vz = pk4(v.x, v.y, v.z, v.w);
+          }
+          sts4(f + FS * k, vx);
+          sts4(f + FS * k + 32, vz);
+          if (kA && (ph & (1u << k))) {
+            lmx = amax(lmx, vx);
+            lmz = amax(lmz, vz);
+          }
+          // to the neighbours: the last two columns to the right, 0 to the left
+          if (ot & (1u << k)) ll_store(hout + (j + k ? j + k + 2 - C : 2) * hcol, vx, tag);
+        };
+        for (;;) {
+          column(0, w0, w1, w2, w3);
+          if (n == 1) break;
+          column(1, w1, w2, w3, w0);
+          if (n == 2) break;
+          column(2, w2, w3, w0, w1);
+          if (n == 3) break;
+          column(3, w3, w0, w1, w2);
+          if (n == 4) break;
+          n -= 4;
+          j += 4;
+          f += 4 * FS;
+          cf += 8;
+          ed += 8;
+          tp += 32;
+          ho += 4 * hstep;
+          ev >>= 4;
+          ot >>= 4;
+          ph >>= 4;
+          src >>= 4;
         }
-#pragma unroll 1
-        for (; j < C - 2; ++j) {
-          column(j, f, cf, ed, tp, hbx, hbz, on & 1u, q[0], q[1], q[2], q[3], hx[0], hz[0]);
-          q[0] = q[1];
-          q[1] = q[2];
-          q[2] = q[3];
-          hx[0] = hx[1];
-          hx[1] = hx[2];
-          hz[0] = hz[1];
-          hz[1] = hz[2];
-          f += 96;
-          cf += 2;
-          ed += 2;
-          tp += 4;
-          on >>= 1;
-          hbx += hstep;
-          hbz += hstep;
+      };
+      for (int j = vj0, je = chi;;) {
+        if (j == 0) {
+          if (je <= 1) fetch();
+          put_left();
+        }
+        if (j == C - 1 && rhalo) {  // the last column is the warp's only one
+          fetch();
+          put_right();
+        }
+        columns(j, je);
+        if (clo > 0 || je <= 1) break;
+        j = 0;  // column 0
+        je = 1;
+        if (kB) {
+          hx[0] = ex;
+          hz[0] = ez;
         }
       }
-      HT ex[3] = {}, ez[3] = {};
-      if (kB) {
-        ex[0] = ldh(hpx, C - 2, lphys);
-        ez[0] = ldh(hpz, C - 2, lphys);
-        ex[1] = ldh(hpx, C - 1, lphys);
-        ez[1] = ldh(hpz, C - 1, lphys);
-        ex[2] = ldh(hpx, 0, lphys);
-        ez[2] = ldh(hpz, 0, lphys);
-      }
-      // the last two columns, with the right neighbour's first two
-      u64 ra = 0ull, rb = 0ull;
-      if (hasr) {
-        const ulonglong2* h = hmine + (size_t)(it & 1) * hpar + hcta;
-        ll_wait2(h + NP, h + 2 * NP, tag, poll, ra, rb);
-      }
-      const u64 ve = column_at(C - 2, q[0], q[1], q[2], ra, ex[0], ez[0]);
-      if (hasr) ll_store(hout, ve, tag);
-      const u64 vf = column_at(C - 1, q[1], q[2], ra, rb, ex[1], ez[1]);
-      if (hasr) ll_store(hout + NP, vf, tag);
-      // column 0, with the left neighbour's last
-      u64 la = 0ull;
-      if (hasl) la = ll_wait1(hmine + (size_t)(it & 1) * hpar - hcta, tag, poll);
-      const u64 v0 = column_at(0, la, P0, P1, P2, ex[2], ez[2]);
-      if (hasl) ll_store(hout + 2 * NP, v0, tag);
       if (kA) {
-        lmx = __reduce_max_sync(kAll, lmx);
-        lmz = __reduce_max_sync(kAll, lmz);
+        const unsigned mx = __reduce_max_sync(kAll, rows ? __float_as_uint(lmx) & 0x7fffffffu : 0u);
+        const unsigned mz = __reduce_max_sync(kAll, rows ? __float_as_uint(lmz) & 0x7fffffffu : 0u);
         if (lane == 0) {
-          WM[16 + warp] = lmx;
-          WM[32 + warp] = lmz;
+          atomicMax(&WM[1], mx);
+          atomicMax(&WM[2], mz);
         }
       }
       if (kB && it < last) {
         const char* hn = hist_at(slot_b(it + 1), 0);
 #pragma unroll
-        for (int u = 0; u < U; ++u) hq[u] = ldh(hn, 2 + u, lsrc);
+        for (int u = 0; u < HR; ++u) hq[u] = ldh(hn, pj0 + u, lsrc);
       }
-    } else {
+    } else if (aux) {
       if (kA) {  // pressure maximum of this step
-        const unsigned m = __reduce_max_sync(kAll, lane < RB ? WM[lane] : 0u);
-        if (lane == 0 && m >= 0x7f800000u) atomicOr(L.err, kErrNonFinite);
+        const unsigned m = WM[0];
+        __syncwarp();
+        if (lane == 0) {
+          WM[0] = 0;
+          if (m >= 0x7f800000u) atomicOr(L.err, kErrNonFinite);
+        }
         if (FP16) {
           u64* sl = L.slots + (size_t)((it & 1) * 2) * gridDim.x + grp * G;
           if (lane == 0) word_store(sl + b, (u64)tag << 32 | m);
@@ -945,11 +1084,12 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
       }
       if (kB && it < last) scales_b(it + 1);
     }
-    __syncthreads();
+    sync_cta();
     if (kA && aux) {  // publish the velocity maxima of this step
-      const unsigned x = __reduce_max_sync(kAll, lane < RB ? WM[16 + lane] : 0u);
-      const unsigned z = __reduce_max_sync(kAll, lane < RB ? WM[32 + lane] : 0u);
+      const unsigned x = WM[1], z = WM[2];
+      __syncwarp();
       if (lane == 0) {
+        WM[1] = WM[2] = 0;
         if (max(x, z) >= 0x7f800000u) atomicOr(L.err, kErrNonFinite);
         if (FP16) {
           u64* sl = L.slots + (size_t)(4 + (it & 1) * 2) * gridDim.x + grp * G;
@@ -957,6 +1097,7 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
           word_store(sl + gridDim.x + b, (u64)tag << 32 | z);
         }
       }
+      __syncwarp();
     }
   }
 
@@ -979,36 +1120,33 @@ __global__ void __launch_bounds__(32 * (kResRowBlocks + 1), 1)
     }
     __syncthreads();
   }
-  if (!aux && (kA || L.save)) {
-    const float ip = kA && FP16 ? SC[0] : 1.f, ix = kA && FP16 ? SC[1] : 1.f,
-                iz = kA && FP16 ? SC[2] : 1.f;
-    for (int j = 0; j < C; ++j) {
-      unsigned t4[4];
-      tm_ld4(TP + 4 * j, t4);
-      tm_wait(t4);
-      const u64 px = pku(t4[0], t4[1]), pz = pku(t4[2], t4[3]), vx = F[96 * j], vz = F[96 * j + 32];
+  if (comp && (kA || L.save)) {
+    const u64 ip = splat(kA && FP16 ? SC[0] : 1.f), ix = splat(kA && FP16 ? SC[1] : 1.f),
+              iz = splat(kA && FP16 ? SC[2] : 1.f);
+    for (int j = clo; j < chi; ++j) {
+      Q4 px, pz;
+      tm_ld(TP + 8 * j, px, pz);
+      const Q4 vx = lds4(F + FS * j), vz = lds4(F + FS * j + 32);
       if (kA) {
         const unsigned on = lphys >> j & 1u;
-        HP::put(hist_at(last - 1, 0) + j * hstep,
-                mul2(mul2(fsm, add2(px, pz)), pk(r0 ? ip : 0.f, r1 ? ip : 0.f)), pol, on);
-        HP::put(hist_at(last - 1, 1) + j * hstep, mul2(vx, pk(r0 ? ix : 0.f, r1 ? ix : 0.f)), pol, on);
-        HP::put(hist_at(last - 1, 2) + j * hstep, mul2(vz, pk(r0 ? iz : 0.f, r1 ? iz : 0.f)), pol, on);
+        const ptrdiff_t o = (ptrdiff_t)(hoff + j * n1h) * kEs;
+        HQ::put(hist_at(last - 1, 0) + o, keep(mul41(add4(px, pz), ip), rows), pol, on);
+        HQ::put(hist_at(last - 1, 1) + o, keep(mul41(vx, ix), rows), pol, on);
+        HQ::put(hist_at(last - 1, 2) + o, keep(mul41(vz, iz), rows), pol, on);
       }
-      if (L.save && c0 + j < g.n2e) {
+      if (L.save && c0 + j < g.n2e && i1 < ld) {
         const size_t o = (size_t)(c0 + j) * ld + i1;
-        *reinterpret_cast<u64*>(S.px + o) = px;
-        *reinterpret_cast<u64*>(S.pz + o) = pz;
-        *reinterpret_cast<u64*>(S.vx + o) = vx;
-        *reinterpret_cast<u64*>(S.vz + o) = vz;
+        sts4(reinterpret_cast<Q4*>(S.px + o), px);
+        sts4(reinterpret_cast<Q4*>(S.pz + o), pz);
+        sts4(reinterpret_cast<Q4*>(S.vx + o), vx);
+        sts4(reinterpret_cast<Q4*>(S.vz + o), vz);
       }
+      __syncwarp();
     }
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  sync_cta();
+  if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*TB), "r"(tcols));
-  }
 }
 
 // Injection tables: one CTA per grid CTA.
@@ -1144,13 +1282,22 @@ size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta) {
   return std::max((size_t)layout(C, RB, inj_pts, inj_m, inj_sta).total, floor_bytes);
 }
 
-int resident_occupancy(int mode, bool fp16, bool rho, int RB, size_t smem) {
+void resident_groups(int C, int RB, int* cg, int* cw) {
+  const int most = RB % 4 ? kResWarps / group_warps(RB) : (kResWarps - 1) / group_warps(RB);
+  *cg = std::max(1, std::min(most, C));
+  *cw = (C + *cg - 1) / *cg;
+  *cg = (C + *cw - 1) / *cw;
+}
+
+int resident_occupancy(int mode, bool fp16, bool rho, int C, int RB, size_t smem) {
   if (smem > kMaxSmem || RB > kResRowBlocks) return 0;
-  int n = 0;
+  int n = 0, cg, cw;
+  resident_groups(C, RB, &cg, &cw);
   with_kernel(mode, fp16, rho, [&](auto k) {
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 32 * (RB + 1), smem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 32 * cta_warps(RB, cg), smem) !=
+            cudaSuccess) {
       cudaGetLastError();
       n = 0;
     }
@@ -1162,7 +1309,10 @@ cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaun
                             bool fp16, cudaStream_t st) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(L.G * L.groups);
-  cfg.blockDim = dim3(32 * (L.RB + 1));
+  ResidentLaunch P = L;
+  P.nz = kNegZero2;
+  resident_groups(L.C, L.RB, &P.CG, &P.CW);
+  cfg.blockDim = dim3(32 * cta_warps(L.RB, P.CG));
   cfg.dynamicSmemBytes = resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -1170,8 +1320,6 @@ cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaun
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  ResidentLaunch P = L;
-  P.nz = kNegZero2;
   cudaError_t e = cudaSuccess;
   with_kernel(mode, fp16, m.rbw1 != nullptr,
               [&](auto k) { e = cudaLaunchKernelEx(&cfg, k, g, m, P); });
