@@ -974,6 +974,18 @@ void gather_boxes(const daw_handle* h, const Batch& b, const ShotCtx& c, int mod
   }
 }
 
+// Quads of rows of the batch's largest rectangles that are staged in shared
+// memory.  A stage of up to kStageBytes takes the stores off the warps that own the
+// rows (2000 of 8700 cycles of their pressure half step on 751 x 2301); taller
+// rectangles are written by their own warps.
+constexpr int kStageBytes = 8 << 10;
+int staged_quads(int C, const Box box[2]) {
+  int q = 0;
+  for (int k = 0; k < 2; ++k)
+    if (box[k].elems()) q += (box[k].r1 - (box[k].r0 & ~3) + 3) / 4;
+  return q * C * 16 <= kStageBytes ? q : 0;
+}
+
 // Columns per CTA with which the batch's runs of `modes` can stay on chip, or
 // 0.  The rule is on the grid (its points fit the SMs' registers and shared
 // memory), on where the stations inject (clear of the rows and columns that
@@ -995,7 +1007,12 @@ int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> m
   for (int C = std::max(4, (g.n2e + h->sms - 1) / h->sms); C <= kResCols; ++C) {
     bool ok = true;
     for (int mode : modes) {
-      int pts = 0, m = 0, nsta = 0;
+      int pts = 0, m = 0, nsta = 0, quads = 0;
+      for (const ShotCtx* c : b.shots) {
+        Box box[2];
+        gather_boxes(h, b, *c, mode, box);
+        quads = std::max(quads, staged_quads(C, box));
+      }
       if (mode == FM_FWD || mode == FM_STAGE_A)
         for (const ShotCtx* c : b.shots) {
           int p1, m1, n1;
@@ -1007,7 +1024,7 @@ int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> m
           nsta = std::max(nsta, n1);
         }
       if (nsta > 60000) return 0;
-      const int occ = resident_occupancy(mode, fp16, rho, C, RB, resident_smem(C, RB, pts, m, nsta));
+      const int occ = resident_occupancy(mode, fp16, rho, C, RB, resident_smem(C, RB, pts, m, nsta, quads));
       ok = ok && occ * h->sms >= (g.n2e + C - 1) / C;
     }
     if (ok) return C;
@@ -1097,8 +1114,19 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
     L.inj_m = std::max(L.inj_m, t.m);
     L.inj_sta = std::max(L.inj_sta, t.nsta);
   }
-  const int occ = resident_occupancy(kmode, fp16, h->md.rbw1 != nullptr, L.C, L.RB,
-                                     resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta));
+  // staged only when every shot's rectangles are
+  bool stage = true;
+  for (const ShotCtx* c : act) {
+    Box box[2];
+    gather_boxes(h, b, *c, mode, box);
+    const int q = staged_quads(L.C, box);
+    stage = stage && (q > 0 || box[0].elems() + box[1].elems() == 0);
+    L.quads = std::max(L.quads, q);
+  }
+  if (!stage) L.quads = 0;
+  const int occ = resident_occupancy(
+      kmode, fp16, h->md.rbw1 != nullptr, L.C, L.RB,
+      resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads));
   const int room = occ * h->sms / L.G;  // shots whose CTAs are resident together
   if (room < 1) throw DawError{DAW_ERR_STATE, "on-chip time loop does not fit"};
   const int q = std::min({room, kResShots, (int)act.size()});
@@ -1111,7 +1139,7 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
   L.halo = static_cast<ulonglong2*>(
       zeroed(h, "resident.halo", 4 * ctas * 3 * L.RB * 64 * sizeof(ulonglong2)));
   L.slots = static_cast<unsigned long long*>(
-      zeroed(h, "resident.slots", 8 * ctas * sizeof(unsigned long long)));
+      zeroed(h, "resident.slots", 72 * ctas * sizeof(unsigned long long)));
   for (size_t g0 = 0; g0 < act.size(); g0 += q) {
     const int n = (int)std::min<size_t>(q, act.size() - g0);
     L.groups = n;
@@ -1169,11 +1197,13 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
           S.amp = c.d_ampT + (w ? (size_t)w->s0 * c.nr : 0);
           S.nsta = c.nr;
         }
+        int quad = 0;
         for (int k = 0; k < 2; ++k) {
           const Box& x = boxes[i][k];
           if (!x.elems()) continue;
-          S.rect[k] = ResidentRect{rect + at, rect_elems, x.c1 - x.c0, x.r0, x.r1, x.c0, x.c1};
+          S.rect[k] = ResidentRect{rect + at, rect_elems, x.c1 - x.c0, x.r0, x.r1, x.c0, x.c1, quad};
           at += x.elems();
+          quad += (x.r1 - (x.r0 & ~3) + 3) / 4;
         }
         if ((mode == FM_FWD || mode == FM_STAGE_B_ES) && c.type_rec == 0) {
           S.wf = c.d_wf;

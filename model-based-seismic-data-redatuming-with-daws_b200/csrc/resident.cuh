@@ -18,6 +18,7 @@ struct ResidentRect {
   float* buf;
   size_t step;
   int ld, r0, r1, c0, c1;
+  int quad0;  // first quad of rows in the shared-memory staging (ResidentLaunch::quads)
 };
 
 // Injection tables of one station map for CTAs of C columns: CTA b's points
@@ -48,19 +49,20 @@ struct ResidentLaunch {
   int C, G, RB, groups;         // columns per CTA, CTAs per shot, 128-row blocks, shots
   int CG, CW;                   // column groups and columns of a group (resident_launch)
   ulonglong2* halo;             // [phase][parity][cta][3][RB * 32][2]
-  unsigned long long* slots;    // [ring of 4][field][cta] (max bits, tag)
+  unsigned long long* slots;    // 72 words a CTA: stage A's maxima and their results
   unsigned tag0;                // step tags of this launch: tag0 + step
   int load, save;               // state from / to global memory (else zero / dropped)
   int slo;                      // pressure source margin (1: final esource)
   int n1h, hist_step0;
   int inj_pts, inj_m, inj_sta;  // shared-memory capacities of the injection tables
+  int quads;                    // quads of rows staged for the rectangles, 0: written directly
   unsigned* err;
   unsigned long long nz;        // (-0, -0), set by resident_launch
   ResidentShot shot[kResShots];
 };
 
 // Dynamic shared memory of a CTA.
-size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta);
+size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta, int quads);
 // Warps of a CTA: column groups and columns per group.
 void resident_groups(int C, int RB, int* cg, int* cw);
 // CTAs per SM of (mode, fp16, density) with that much shared memory; 0 when it does not fit.

@@ -44,12 +44,12 @@
 // instructions per lane quad and half step, 46 of them arithmetic), for narrow
 // ones the exchange latency (about 0.5 us per half step).  Tried and slower: the fields in
 // registers with all columns unrolled (30 us a step against 14: instruction
-// cache), lanes of two rows (13.2-14.0 us against 9.2-12.5: the same number of
+// cache), lanes of two rows (13.2-14.0 us against 9.2-12.5 then: the same number of
 // instructions per lane), a separate copy of the column code for the edges.
 // Measured per shot step against the split kernels (B200, FP16 histories):
-// 751 x 2301 (17 columns a CTA) forward 9.2 us against 20.1, stage A 12.5
-// against 20.7-23.0, stage B 9.7 against 19.7-24.7; 151 x 461 (4 columns)
-// 2.4-6.2 us against 12-15.
+// 751 x 2301 (17 columns a CTA) forward 7.1 us against 20.1, stage A 10.8
+// against 20.7-23.0, stage B 9.1 against 19.7-24.7; 151 x 461 (4 columns)
+// 2.4-4.0 us against 12-15.
 #include "resident.cuh"
 #include "tma.cuh"
 
@@ -196,12 +196,40 @@ __device__ __forceinline__ unsigned group_max(const u64* s, int G, unsigned tag,
         ok = ok && (unsigned)(v[k] >> 32) == tag;
       }
       if (w.dead || __all_sync(kAll, ok) || w.give_up(n)) break;
-      __nanosleep(100);  // leaves the issue slots to the other warps
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) m = max(m, (unsigned)v[k]);
   }
   return __reduce_max_sync(kAll, m);
+}
+
+// Two maxima over the group's CTAs, by the extra warps: every CTA has stored
+// its tagged words at s and s + stride; the leader collects them and stores the
+// results to each CTA's own line at r.  (All CTAs polling all words made the lines
+// they share the bottleneck: 3 us an exchange with 126 CTAs.)
+constexpr int kLine = 16;  // words of a 128-byte line
+__device__ __forceinline__ uint2 exchange_max(const u64* s, size_t stride, int fields, u64* r, int b,
+                                              int G, int leader, unsigned tag, Poll& w) {
+  const int lane = threadIdx.x & 31;
+  uint2 m = make_uint2(0u, 0u);
+  if (b == leader) {
+    m.x = group_max(s, G, tag, w);
+    if (fields > 1) m.y = group_max(s + stride, G, tag, w);
+    for (int i = lane; i < G; i += 32) {
+      word_store(r + (size_t)i * kLine, (u64)tag << 32 | m.x);
+      word_store(r + (size_t)i * kLine + 1, (u64)tag << 32 | m.y);
+    }
+    return m;
+  }
+  const u64* own = r + (size_t)b * kLine + (lane & 1);
+  u64 v;
+  for (int n = 0;; ++n) {
+    v = word_load(own);
+    if (w.dead || __all_sync(kAll, (unsigned)(v >> 32) == tag) || w.give_up(n)) break;
+  }
+  m.x = __shfl_sync(kAll, (unsigned)v, 0);
+  m.y = __shfl_sync(kAll, (unsigned)v, 1);
+  return m;
 }
 
 // The history of a lane's four rows: FP16 in 64 bits, FP32 in 128.  Loads and
@@ -263,6 +291,12 @@ __device__ __forceinline__ void sts_if(u64* p, u64 v, unsigned on) {
   asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p st.shared.b64 [%0], %1;\n}" ::"r"(
                    smem_u32(p)),
                "l"(v), "r"(on)
+               : "memory");
+}
+__device__ __forceinline__ void sts_if(Q4* p, Q4 v, unsigned on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.shared.v2.b64 [%0], {%1, %2};\n}" ::"r"(
+                   smem_u32(p)),
+               "l"(v.a), "l"(v.b), "r"(on)
                : "memory");
 }
 __device__ __forceinline__ void lds_if(float& v, const float* p, unsigned on) {
@@ -344,9 +378,9 @@ __device__ __forceinline__ void sync_cta() {
 
 // Shared-memory layout (offsets in bytes, 16-byte aligned sections).
 struct Lay {
-  int fld, halo, edge, col, row, tcd, term, tsta, tkap, amp, misc, total;
+  int fld, halo, edge, col, row, tcd, term, tsta, tkap, amp, stage, misc, total;
 };
-__host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta) {
+__host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, int quads) {
   Lay l;
   int o = 0;
   auto take = [&](int bytes) {
@@ -366,6 +400,7 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta) {
   l.tsta = take(pts * m * 2);
   l.tkap = take(pts * 4);
   l.amp = take((nsta + 1) * 4);
+  l.stage = take(quads * C * 16);    // pressure of the gather rectangles [quad][column]
   l.misc = take(64 * 4 + 16);
   l.total = o;
   return l;
@@ -389,15 +424,15 @@ __host__ __device__ inline int aux_warp(int RB, int CG) {
   return RB % 4 ? RB : CG * group_warps(RB);
 }
 
-// The injection terms ((c dt) amp) kappa of one step, by all warps.
-__device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int pts, int m) {
+// The injection terms ((c dt) amp) kappa of one step, by thread t of nt.
+__device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int pts, int m, int t, int nt) {
   const float2* cd = reinterpret_cast<const float2*>(sm + l.tcd);
   float2* term = reinterpret_cast<float2*>(sm + l.term);
   const ushort2* sta = reinterpret_cast<const ushort2*>(sm + l.tsta);
   const float* kap = reinterpret_cast<const float*>(sm + l.tkap);
   const float* amp = reinterpret_cast<const float*>(sm + l.amp);
   const int mh = m / 2;
-  for (int p = threadIdx.x; p < pts; p += blockDim.x) {
+  for (int p = t; p < pts; p += nt) {
     const float kv = kap[p];
     for (int k = 0; k < mh; ++k) {
       const float2 c = cd[p * mh + k];
@@ -418,7 +453,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   using HT = typename HQ::T;
   extern __shared__ __align__(16) unsigned char sm[];
   const int C = L.C, G = L.G, RB = L.RB;
-  const Lay l = layout(C, RB, L.inj_pts, L.inj_m, L.inj_sta);
+  const Lay l = layout(C, RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads);
   const int grp = blockIdx.x / G, b = blockIdx.x - grp * G;
   const ResidentShot& S = L.shot[grp];
   // the warp index from a shuffle: the compiler then knows that it, and all
@@ -431,7 +466,9 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   const int npml = g.npml, ld = g.ld;
   const int first = S.first, last = S.last;
   if (first > last) return;             // uniform over the group
-  const int clo = cg * L.CW, chi = min(C, clo + L.CW);  // the warp's columns
+  // the warp's columns; the first group, whose edge costs more, has those left over
+  const int over = L.CG * L.CW - C;
+  const int clo = max(cg * L.CW - over, 0), chi = min(C, cg * L.CW + L.CW - over);
   // the lane's vx, vz of column j: F[FS j], F[FS j + 32]; the vz pair above and the row below it at FU, FD (lanes 0 and 31: in the
   // neighbouring row blocks; the grid's first and last rows, which are never
   // updated, stand for the zeros beyond them)
@@ -570,7 +607,9 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
     }
   }
   __syncthreads();
-  if (ipts > 0) inj_terms(sm, l, ipts, im);
+  // the warps but the extra one
+  const int it0 = tid - (warp > aux_warp(RB, L.CG) ? 32 : 0), itn = blockDim.x - 32;
+  if (ipts > 0 && !aux) inj_terms(sm, l, ipts, im, it0, itn);
 
   const u64 nz = L.nz;
   auto mul2 = [&](u64 x, u64 y) { return fma2(x, y, nz); };
@@ -618,20 +657,34 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   const bool hasl = b > 0, hasr = b + 1 < G;
   const bool inj_on = ipts > 0 && comp && i1 + 3 >= ih.x && i1 < ih.x + ih.y;
   const bool inj_warp = !kB && ipts > 0 && comp && 128 * rb + 127 >= ih.x && 128 * rb < ih.x + ih.y;
-  // rectangles kept for the gathers: the CTA's columns, the lane's rows and the
-  // address of its first row and the CTA's first column at the current step
-  unsigned rcol[2] = {}, rrow[2] = {};
+  // Rectangles kept for the gathers.  With room in shared memory (L.quads) the
+  // lanes put their quads there and the extra warp writes them to memory during
+  // the velocity half step, a row's columns together; else the lanes write their
+  // rows: the lane's rows and the address of its first row and the CTA's first
+  // column at the current step.
+  unsigned rcol[2] = {}, rrow[2] = {};  // written by the lanes: the CTA's columns, the lane's rows
   float* rptr[2] = {};
+  Q4* const stage = reinterpret_cast<Q4*>(sm + l.stage);
+  const bool staged = !kA && L.quads > 0;
+  Q4* sptr[2] = {stage, stage};
+  unsigned son[2] = {};  // staged: the lane's quad is one of the rectangle's
   if (!kA && comp)
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const ResidentRect& R = S.rect[q];
       if (!R.buf || 128 * rb + 127 < R.r0 || 128 * rb >= R.r1) continue;
-      const int a = max(R.c0 - c0, 0), e = min(R.c1 - c0, C);
-      rcol[q] = e > a ? (1u << e) - (1u << a) : 0u;
+      unsigned rows4 = 0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) rrow[q] |= (i1 + k >= R.r0 && i1 + k < R.r1 ? 1u : 0u) << k;
-      rptr[q] = R.buf + (ptrdiff_t)(i1 - R.r0) * R.ld + (c0 - R.c0);
+      for (int k = 0; k < 4; ++k) rows4 |= (i1 + k >= R.r0 && i1 + k < R.r1 ? 1u : 0u) << k;
+      if (staged) {
+        son[q] = rows4;
+        if (rows4) sptr[q] = stage + (R.quad0 + (i1 - (R.r0 & ~3)) / 4) * C;
+      } else {
+        const int a = max(R.c0 - c0, 0), e = min(R.c1 - c0, C);
+        rcol[q] = e > a ? (1u << e) - (1u << a) : 0u;
+        rrow[q] = rows4;
+        rptr[q] = R.buf + (ptrdiff_t)(i1 - R.r0) * R.ld + (c0 - R.c0);
+      }
     }
   // warps with more to do per column than the update (warp-uniform)
   const bool extra = !kA && comp && ((rcol[0] | rcol[1]) != 0 || S.wf != nullptr);
@@ -681,6 +734,13 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       for (int u = 0; u < HR; ++u) hq[u] = ldh(hist_at(slot_b(first), 0), pj0 + u, lsrc);
     }
   }
+  // stage A: the lines of the exchanged maxima, [phase][parity][cta], and the
+  // CTA that collects the velocities' (the pressure's: CTA 0)
+  const int vleader = G / 2;
+  auto results = [&](int phase, int s) {
+    return L.slots + (size_t)8 * gridDim.x +
+           ((size_t)(phase * 2 + (s & 1)) * gridDim.x + grp * G) * kLine;
+  };
   sync_cta();
 
   for (int it = first; it <= last; ++it) {
@@ -733,6 +793,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         unsigned tp = TP + 8 * j, tk = TK + 4 * j, ho = (unsigned)((hoff + j * n1h) * kEs);
         unsigned ev = events >> j, ot = outs >> j, ph = phys >> j, src = lsrc >> j;
         int n = je - j;
+        Q4 *sp0 = sptr[0] + j, *sp1 = sptr[1] + j;
         Q4 w0 = lds4(f - 2 * FS), w1 = lds4(f - FS), w2 = lds4(f), w3;
         auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
           if (ev & (1u << k)) {
@@ -762,15 +823,22 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           if (inj_warp) {
             if (inj_on) {  // the lane's four rows are rows of the table
               float4 v = up4(px);
-              const float2* t =
-                  reinterpret_cast<const float2*>(TERM + ((j + k) * ih.y + (i1 - ih.x)) * im);
-              const int mh = im >> 1;
+              const float* t0 = TERM + ((j + k) * ih.y + (i1 - ih.x)) * im;
+              const float2* t = reinterpret_cast<const float2*>(t0);
+              // a forward run's map has one station: one term a point
+              const int mh = kF ? 0 : im >> 1;
+              if (kF) {
+                v.x = fadd(v.x, t0[0]);
+                v.y = fadd(v.y, t0[im]);
+                v.z = fadd(v.z, t0[2 * im]);
+                v.w = fadd(v.w, t0[3 * im]);
+              }
               for (int q = 0; q < mh; ++q) {
                 const float2 a = t[q], e = t[mh + q], c = t[2 * mh + q], d = t[3 * mh + q];
-                v.x = kA ? fsub(fsub(v.x, a.x), a.y) : fadd(fadd(v.x, a.x), a.y);
-                v.y = kA ? fsub(fsub(v.y, e.x), e.y) : fadd(fadd(v.y, e.x), e.y);
-                v.z = kA ? fsub(fsub(v.z, c.x), c.y) : fadd(fadd(v.z, c.x), c.y);
-                v.w = kA ? fsub(fsub(v.w, d.x), d.y) : fadd(fadd(v.w, d.x), d.y);
+                v.x = fsub(fsub(v.x, a.x), a.y);
+                v.y = fsub(fsub(v.y, e.x), e.y);
+                v.z = fsub(fsub(v.z, c.x), c.y);
+                v.w = fsub(fsub(v.w, d.x), d.y);
               }
               px = pk4(v.x, v.y, v.z, v.w);
             }
@@ -787,6 +855,10 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           sts_if(ed + 2 * k, p.a, top);
           sts_if(ed + 2 * k + 1, p.b, bottom);
           if (kA && (ph & (1u << k))) lmax = amax(lmax, p);
+          if (!kA) {  // no branch: its code would be cold for the few warps that take it
+            sts_if(sp0 + k, p, son[0]);
+            sts_if(sp1 + k, p, son[1]);
+          }
           if (extra) {
             // pressure rows of the gather rectangles, and the wavefield output
             const float4 v = up4(p);
@@ -818,6 +890,8 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           j += 4;
           f += 4 * FS;
           fu += 8 * FS;
+          sp0 += 4;
+          sp1 += 4;
           fd += 16 * FS;
           cf += 8;
           ed += 8;
@@ -858,13 +932,11 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         }
       }
     } else if (aux) {
-      if (!kB && ipts > 0 && it < last)  // amplitudes of the next step
-        for (int k = lane; k < ih.w; k += 32) AMP[k] = S.amp[(size_t)it * S.nsta + ih.z + k];
       if (kA && it > first) {            // velocity maxima of the previous step
         if (FP16) {
-          u64* sl = L.slots + (size_t)(4 + ((it - 1) & 1) * 2) * gridDim.x + grp * G;
-          const unsigned vx = group_max(sl, G, tag - 1, poll);
-          const unsigned vz = group_max(sl + gridDim.x, G, tag - 1, poll);
+          const uint2 m = exchange_max(L.slots + (size_t)(4 + ((it - 1) & 1) * 2) * gridDim.x + grp * G,
+                                       gridDim.x, 2, results(1, it - 1), b, G, vleader, tag - 1, poll);
+          const unsigned vx = m.x, vz = m.y;
           if (lane == 0) {
             SC[1] = pow2f(15 - amax_exponent(vx));
             SC[2] = pow2f(15 - amax_exponent(vz));
@@ -876,6 +948,8 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           }
         }
       }
+      if (!kB && ipts > 0 && it < last)  // amplitudes of the next step
+        for (int k = lane; k < ih.w; k += 32) AMP[k] = S.amp[(size_t)it * S.nsta + ih.z + k];
       if (kB) prefetch_b(it + 2);
     }
     if (extra) {
@@ -884,7 +958,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
     }
     sync_cta();
     // =============== velocity half step ===============
-    if (!kB && ipts > 0 && it < last) inj_terms(sm, l, ipts, im);
+    if (!kB && ipts > 0 && it < last && !aux) inj_terms(sm, l, ipts, im, it0, itn);
     if (comp) {
       const Q4 d1b = lds4(ROW + 2 * NP), bw1 = lds4(ROW + 3 * NP);
       const u64 INVX = splat(kA && FP16 ? SC[1] : 1.f), INVZ = splat(kA && FP16 ? SC[2] : 1.f);
@@ -1075,12 +1149,27 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         if (FP16) {
           u64* sl = L.slots + (size_t)((it & 1) * 2) * gridDim.x + grp * G;
           if (lane == 0) word_store(sl + b, (u64)tag << 32 | m);
-          const unsigned p = group_max(sl, G, tag, poll);
+          const unsigned p = exchange_max(sl, 0, 1, results(0, it), b, G, 0, tag, poll).x;
           if (lane == 0) {
             SC[0] = pow2f(15 - amax_exponent(p));
             if (b == 0) S.amax[(size_t)(it - 1) * 3 * kAmaxSlots] = p;
           }
         }
+      }
+      if (staged) {
+        const int c = c0 + lane;
+        for (int q = 0; q < 2; ++q) {
+          const ResidentRect& R = S.rect[q];
+          if (!R.buf || lane >= C || c < R.c0 || c >= R.c1) continue;
+          const float* v = reinterpret_cast<const float*>(stage + R.quad0 * C + lane);
+          float* o = R.buf + (size_t)(it - first) * R.step + (c - R.c0);
+#pragma unroll 4
+          for (int r = R.r0; r < R.r1; ++r) {
+            const int k = r - (R.r0 & ~3);
+            o[(ptrdiff_t)(r - R.r0) * R.ld] = v[(k >> 2) * 4 * C + (k & 3)];
+          }
+        }
+        __syncwarp();
       }
       if (kB && it < last) scales_b(it + 1);
     }
@@ -1105,9 +1194,9 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   if (kA) {
     if (aux && FP16) {
       const unsigned tag = L.tag0 + (unsigned)last;
-      u64* sl = L.slots + (size_t)(4 + (last & 1) * 2) * gridDim.x + grp * G;
-      const unsigned vx = group_max(sl, G, tag, poll);
-      const unsigned vz = group_max(sl + gridDim.x, G, tag, poll);
+      const uint2 m = exchange_max(L.slots + (size_t)(4 + (last & 1) * 2) * gridDim.x + grp * G,
+                                   gridDim.x, 2, results(1, last), b, G, vleader, tag, poll);
+      const unsigned vx = m.x, vz = m.y;
       if (lane == 0) {
         SC[1] = pow2f(15 - amax_exponent(vx));
         SC[2] = pow2f(15 - amax_exponent(vz));
@@ -1271,7 +1360,7 @@ constexpr int kTmCols = 512;
 
 }  // namespace
 
-size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta) {
+size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta, int quads) {
   const int tw = tm_words(C, RB);
   if (tw > kTmCols) return kMaxSmem + 1;
   // No more CTAs may be resident on an SM than its tensor memory holds: shared
@@ -1279,7 +1368,7 @@ size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta) {
   // fit would block inside the kernel).
   const size_t n = kTmCols / tm_alloc(C, RB);
   const size_t floor_bytes = kMaxSmem / (n + 1) + 128;
-  return std::max((size_t)layout(C, RB, inj_pts, inj_m, inj_sta).total, floor_bytes);
+  return std::max((size_t)layout(C, RB, inj_pts, inj_m, inj_sta, quads).total, floor_bytes);
 }
 
 void resident_groups(int C, int RB, int* cg, int* cw) {
@@ -1313,7 +1402,7 @@ cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaun
   P.nz = kNegZero2;
   resident_groups(L.C, L.RB, &P.CG, &P.CW);
   cfg.blockDim = dim3(32 * cta_warps(L.RB, P.CG));
-  cfg.dynamicSmemBytes = resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta);
+  cfg.dynamicSmemBytes = resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;  // CTAs wait on one another: all are resident
