@@ -27,7 +27,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp-contract=off",
           f"-I{INCLUDE}", f"-I{CSRC}"]
 LIB_SOURCES = ["hicks.cpp", "engine.cu", "stencil_plain.cu", "stencil_fused.cu", "stencil_tma.cu", "stencil_step.cu",
-               "stencil_resident.cu",
+               "stencil_resident.cu", "tables.cu",
                "minres.cu",
                "filter.cu", "filter_noalloc.cu", "driver.cpp"]
 

@@ -25,6 +25,8 @@ constexpr int kNAlpha = 100;       // sub-grid positions per axis (nalpha)
 // 21x21 monopole tile of one station, tile[(i1+10) + 21*(i2+10)], with the
 // free-surface anti-mirroring for nalpha_frees > 0.
 void hicks_tile(int ialpha1, int ialpha2, int nfs, float* tile);
+// The 1-D weights behind it, [21 taps][100 positions].
+const float* hicks_weights();
 // subsourcekws for a 2-D position (z, x): out5 = ix1, ix2 (1-based, physical),
 // ialpha1, ialpha2, nalpha_frees.
 void hicks_locate(float z, float x, float h, int ofs, int32_t out5[5]);
@@ -93,7 +95,9 @@ struct StationsDev {
 
 // Gather-form injection map of a station set on the extended grid: for every
 // touched grid point the (station, coefficient) contributions in station
-// order, so the per-point sum has the reference's accumulation order.
+// order, so the per-point sum has the reference's accumulation order.  pt, ptr,
+// sta and coef are null in a map built on the device (the plain and the register
+// kernels read them).
 struct InjMapDev {
   int npts = 0, nent = 0;
   int* pt = nullptr;       // linear index i1 + ld*i2 (0-based) of each touched point

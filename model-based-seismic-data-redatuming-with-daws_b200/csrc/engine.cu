@@ -137,7 +137,10 @@ void sponge_b(int npml, int n, std::vector<float>& d, std::vector<float>& d1) {
 // the touched rows (lo > hi: none), the most entries of a point and the range
 // of its stations, and the bounding box of all touched points.
 struct MapInfo {
-  std::vector<int> lo, hi, cnt, smin, smax;
+  std::vector<int> cols;  // lo, hi and the dense index of row lo, n2e each
+  std::vector<int> cnt, smin, smax;
+  const int *lo = nullptr, *hi = nullptr;  // into cols
+  int rows = 0, most = 0, entries = 0;     // dense rows, most entries of a point, all entries
   int r0 = INT_MAX, r1 = -1, c0 = INT_MAX, c1 = -1;  // inclusive; r1 < r0: empty
 };
 
@@ -159,6 +162,7 @@ struct ShotCtx {
   StationsDev rec, src;
   InjMapDev recmap, srcmap;
   MapInfo recinfo, srcinfo;
+  std::vector<int32_t> rec_table;  // host copy of the receivers' table
   ResTables rectab, srctab;
   float *d_s = nullptr, *d_dobs = nullptr, *d_datar = nullptr, *d_deltadr = nullptr;
   float *d_deltade = nullptr, *d_dataesc = nullptr, *d_datae = nullptr;
@@ -251,6 +255,7 @@ struct daw_handle {
     float us_per_step;     // measured device time of one step per shot (0: not measured)
   };
   std::map<std::string, Tuned> tuned;
+  float* d_weights = nullptr;  // 1-D Hicks weights [tap][position]
   unsigned res_tag = 1;  // next step tag of the on-chip time loops
 };
 
@@ -297,31 +302,107 @@ void check_table(const daw_handle* h, const int32_t* tab, int n, bool extended, 
   }
 }
 
+// Stations of a table; `tab` stays valid until the stream has been synchronised.
 StationsDev make_stations(daw_handle* h, Pool& pool, const std::string& name, const int32_t* tab,
                           int n) {
   StationsDev s;
   s.n = n;
   if (n == 0) return s;
-  std::vector<int> ix1(n), ix2(n);
-  std::vector<float> tiles((size_t)n * kTile);
-  for (int i = 0; i < n; ++i) {
-    ix1[i] = tab[i];
-    ix2[i] = tab[i + n];
-    hicks_tile(tab[i + 2 * n], tab[i + 3 * n], tab[i + 4 * n], tiles.data() + (size_t)i * kTile);
-  }
+  int* dt = pool.get_t<int>(name + ".tab", (size_t)n * 5);
   s.ix1 = pool.get_t<int>(name + ".ix1", n);
   s.ix2 = pool.get_t<int>(name + ".ix2", n);
   s.tile = pool.get_t<float>(name + ".tile", (size_t)n * kTile);
-  upload(s.ix1, ix1.data(), n * sizeof(int), h->st);
-  upload(s.ix2, ix2.data(), n * sizeof(int), h->st);
-  upload(s.tile, tiles.data(), tiles.size() * sizeof(float), h->st);
-  sync(h);  // host vectors go out of scope
+  upload(dt, tab, (size_t)n * 5 * sizeof(int), h->st);
+  station_tiles(dt, n, h->d_weights, s, h->st);
+  check_launch("station tiles");
+  h->tim.kernel_launches += 1;
   return s;
 }
 
-// Gather-form injection map of stations `tab` on the extended grid.
+// Touched rows, entry counts and station ranges of the stations' supports.
+void map_info(const Grid& g, const int32_t* tab, int n, MapInfo* m) {
+  *m = MapInfo();
+  std::vector<int> &cols = m->cols;
+  cols.assign((size_t)3 * g.n2e, 0);
+  int *lo = cols.data(), *hi = lo + g.n2e, *base = hi + g.n2e;
+  std::fill(lo, lo + g.n2e, INT_MAX);
+  std::fill(hi, hi + g.n2e, -1);
+  m->lo = lo;
+  m->hi = hi;
+  m->cnt.assign(g.n2e, 0);
+  m->smin.assign(g.n2e, INT_MAX);
+  m->smax.assign(g.n2e, -1);
+  std::vector<std::vector<int>> of(g.n2e);  // stations of each column
+  for (int s = 0; s < n; ++s) {
+    const int a0 = std::max(tab[s] - 1 - kRad, 0), a1 = std::min(tab[s] - 1 + kRad, g.n1e - 1);
+    const int b0 = std::max(tab[s + n] - 1 - kRad, 0), b1 = std::min(tab[s + n] - 1 + kRad, g.n2e - 1);
+    if (a0 > a1 || b0 > b1) continue;
+    m->entries += (a1 - a0 + 1) * (b1 - b0 + 1);
+    m->r0 = std::min(m->r0, a0);
+    m->r1 = std::max(m->r1, a1);
+    m->c0 = std::min(m->c0, b0);
+    m->c1 = std::max(m->c1, b1);
+    for (int c = b0; c <= b1; ++c) {
+      lo[c] = std::min(lo[c], a0);
+      hi[c] = std::max(hi[c], a1);
+      m->smin[c] = std::min(m->smin[c], s);
+      m->smax[c] = std::max(m->smax[c], s);
+      of[c].push_back(s);
+    }
+  }
+  std::vector<int> diff;
+  for (int c = 0; c < g.n2e; ++c) {
+    base[c] = m->rows;
+    if (hi[c] < lo[c]) continue;
+    m->rows += hi[c] - lo[c] + 1;
+    // most stations over one row: a sweep over the rows where supports begin and end
+    diff.assign(hi[c] - lo[c] + 2, 0);
+    for (int s : of[c]) {
+      const int a0 = std::max(tab[s] - 1 - kRad, 0), a1 = std::min(tab[s] - 1 + kRad, g.n1e - 1);
+      ++diff[a0 - lo[c]];
+      --diff[a1 + 1 - lo[c]];
+    }
+    int k = 0;
+    for (int d : diff) {
+      k += d;
+      m->cnt[c] = std::max(m->cnt[c], k);
+    }
+    m->most = std::max(m->most, m->cnt[c]);
+  }
+}
+
+// The injection map for the TMA kernels and the on-chip loops, built on the
+// device with `most` entry slots per point (info must outlive the next
+// synchronisation).  The full map, with the arrays of the plain and register
+// kernels (and without empty slots), comes from make_full_map.
+InjMapDev make_full_map(daw_handle* h, Pool& pool, const std::string& name, const int32_t* tab, int n);
+bool tma_path(const daw_handle* h);
 InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int32_t* tab, int n,
-                   MapInfo* info) {
+                   const StationsDev& st, MapInfo* info) {
+  const Grid& g = h->g;
+  map_info(g, tab, n, info);
+  const size_t slots = (size_t)info->rows * info->most;
+  // a map whose points have very different entry counts would be mostly empty slots
+  if (!tma_path(h) || slots > (size_t)8 * info->entries + 1024 || slots > (1u << 30))
+    return make_full_map(h, pool, name, tab, n);
+  InjMapDev m;
+  m.nent = info->entries;
+  m.nsta = n;
+  int* cols = pool.get_t<int>(name + ".cols", (size_t)3 * g.n2e);
+  m.col_lo = cols;
+  m.col_hi = cols + g.n2e;
+  m.col_base = cols + 2 * g.n2e;
+  m.rowptr = pool.get_t<int>(name + ".rp", std::max<size_t>(2, (size_t)2 * info->rows));
+  m.ent = pool.get_t<float2>(name + ".ent", std::max<size_t>(1, slots));
+  upload(cols, info->cols.data(), info->cols.size() * sizeof(int), h->st);
+  injection_map(st, g.n2e, info->most, m, h->st);
+  check_launch("injection map");
+  h->tim.kernel_launches += 1;
+  return m;
+}
+
+// Gather-form injection map of stations `tab` on the extended grid.
+InjMapDev make_full_map(daw_handle* h, Pool& pool, const std::string& name, const int32_t* tab, int n) {
   const Grid& g = h->g;
   struct E {
     long long pt;
@@ -407,21 +488,6 @@ InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int
       if (chi[c] >= clo[c]) idx += chi[c] - clo[c] + 1;
     }
   }
-  info->lo = clo;
-  info->hi = chi;
-  info->cnt.assign(g.n2e, 0);
-  info->smin.assign(g.n2e, INT_MAX);
-  info->smax.assign(g.n2e, -1);
-  for (size_t q = 0; q < pt.size(); ++q) {
-    const int c = pt[q] / g.ld, r = pt[q] % g.ld;
-    info->cnt[c] = std::max(info->cnt[c], ptr[q + 1] - ptr[q]);
-    info->smin[c] = std::min(info->smin[c], sta[ptr[q]]);  // entries are in station order
-    info->smax[c] = std::max(info->smax[c], sta[ptr[q + 1] - 1]);
-    info->r0 = std::min(info->r0, r);
-    info->r1 = std::max(info->r1, r);
-    info->c0 = std::min(info->c0, c);
-    info->c1 = std::max(info->c1, c);
-  }
   InjMapDev m;
   m.npts = (int)pt.size();
   m.nent = (int)sta.size();
@@ -432,7 +498,7 @@ InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int
   m.col_lo = pool.get_t<int>(name + ".clo", g.n2e);
   m.col_hi = pool.get_t<int>(name + ".chi", g.n2e);
   m.col_base = pool.get_t<int>(name + ".cbase", g.n2e);
-  m.rowptr = pool.get_t<int>(name + ".rp", std::max<size_t>(2, rp.size()));
+  m.rowptr = pool.get_t<int>(name + ".frp", std::max<size_t>(2, rp.size()));
   upload(m.pt, pt.data(), pt.size() * sizeof(int), h->st);
   upload(m.ptr, ptr.data(), ptr.size() * sizeof(int), h->st);
   upload(m.sta, sta.data(), sta.size() * sizeof(int), h->st);
@@ -447,7 +513,7 @@ InjMapDev make_map(daw_handle* h, Pool& pool, const std::string& name, const int
     std::memcpy(&sbits, &sta[i], sizeof sbits);
     ent[i] = make_float2(coef[i], sbits);
   }
-  m.ent = pool.get_t<float2>(name + ".ent", std::max<size_t>(1, ent.size()));
+  m.ent = pool.get_t<float2>(name + ".fent", std::max<size_t>(1, ent.size()));
   upload(m.ent, ent.data(), ent.size() * sizeof(float2), h->st);
   m.nsta = n;
   sync(h);
@@ -1432,7 +1498,19 @@ void clear_amax(daw_handle* h, Batch& b) {
 // ---------------------------------------------------------------------------
 // Operators over a batch.  op_in/op_out/op_reverse are set per shot.
 // ---------------------------------------------------------------------------
+// The plain and the register kernels read the full maps.
+void full_maps(daw_handle* h, Batch& b, bool source) {
+  if (tma_path(h)) return;
+  for (ShotCtx* c : b.shots) {
+    InjMapDev& m = source ? c->srcmap : c->recmap;
+    if (m.ptr) continue;
+    m = source ? make_full_map(h, h->pool, c->tag + "srcmap", c->src5, 1)
+               : make_full_map(h, h->pool, c->tag + "recmap", c->rec_table.data(), c->nr);
+  }
+}
+
 void batch_forward(daw_handle* h, Batch& b) {
+  full_maps(h, b, true);
   if (!h->opt.fused) {
     for (ShotCtx* c : b.shots)
       plain_forward(h, *c, c->d_datar, c->d_wf, h->ndatum && !b.no_datum ? c->d_redF : nullptr);
@@ -1526,6 +1604,7 @@ void shot_operator_windowed(daw_handle* h, Batch& b, bool esource) {
 // Stage A + stage B.  esource: final simulation (interior 2..n-1 pressure
 // source, datum gather, optional wavefield accumulation and cost).
 void batch_operator(daw_handle* h, Batch& b, bool esource) {
+  full_maps(h, b, false);
   if (!h->opt.fused) {
     for (ShotCtx* c : b.shots) {
       if (!c->active) continue;
@@ -1881,11 +1960,11 @@ void prepare_shot(daw_handle* h, ShotCtx& c, const daw_shot_desc& d, int slot, b
   upload(c.d_s, d.s, (size_t)d.nt * 4, h->st);
   if (d.dobs) upload(c.d_dobs, d.dobs, n * 4, h->st);
   c.rec = make_stations(h, h->pool, p + "rec", d.rec_tab, d.nrec);
-  c.recmap = make_map(h, h->pool, p + "recmap", d.rec_tab, d.nrec, &c.recinfo);
-  int32_t s5[5];
-  std::memcpy(s5, d.src_tab, sizeof s5);
-  c.src = make_stations(h, h->pool, p + "src", s5, 1);
-  c.srcmap = make_map(h, h->pool, p + "srcmap", s5, 1, &c.srcinfo);
+  c.rec_table.assign(d.rec_tab, d.rec_tab + (size_t)5 * d.nrec);
+  c.recmap = make_map(h, h->pool, p + "recmap", d.rec_tab, d.nrec, c.rec, &c.recinfo);
+  c.src = make_stations(h, h->pool, p + "src", c.src5, 1);
+  c.srcmap = make_map(h, h->pool, p + "srcmap", c.src5, 1, c.src, &c.srcinfo);
+  sync(h);  // the descriptor's arrays have been read
   c.d_wf = want_wf ? h->pool.get_t<float>(p + "wf", g.int_elems() * (size_t)d.nt) : nullptr;
   c.d_ampT = h->pool.get_t<float>(p + "ampT", std::max<size_t>(n, 1));
   // forward-only shots keep no history: one step is allocated so that the
@@ -2201,7 +2280,8 @@ ShotCtx& single_ctx(daw_handle* h, ShotCtx& c, int nt, const int32_t* ir, int nr
   c.d_redF = a + 7 * n; c.d_redE = c.d_redF + nd; c.d_red = c.d_redE + nd; c.d_redf = c.d_red + nd;
   c.d_s = c.d_redf + nd + nd;
   c.rec = make_stations(h, h->pool, p + "rec", ir, nr);
-  c.recmap = make_map(h, h->pool, p + "recmap", ir, nr, &c.recinfo);
+  c.rec_table.assign(ir, ir + (size_t)5 * nr);
+  c.recmap = make_map(h, h->pool, p + "recmap", ir, nr, c.rec, &c.recinfo);
   c.d_wf = want_wf ? h->pool.get_t<float>(p + "wf", h->g.int_elems() * (size_t)nt) : nullptr;
   c.d_ampT = h->pool.get_t<float>(p + "ampT", std::max<size_t>(n, 1));
   const int win = forward_only ? 0 : history_window(h, nt, nr, want_wf, admission_bytes(h));
@@ -2289,7 +2369,10 @@ int daw_create(daw_handle** out, int32_t device) {
   if (filter_noalloc_prepare(nullptr, 0) != DAW_OK) cudaGetLastError();
   if (cudaMalloc(&h->d_err, sizeof(unsigned)) != cudaSuccess ||
       cudaMemset(h->d_err, 0, sizeof(unsigned)) != cudaSuccess ||
-      cudaMalloc(&h->d_qctr, 2 * sizeof(unsigned)) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+      cudaMalloc(&h->d_qctr, 2 * sizeof(unsigned)) != cudaSuccess ||
+      cudaMalloc(&h->d_weights, kTap * kNAlpha * sizeof(float)) != cudaSuccess ||
+      cudaMemcpy(h->d_weights, hicks_weights(), kTap * kNAlpha * sizeof(float),
+                 cudaMemcpyHostToDevice) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
     cudaGetLastError();
     cudaStreamDestroy(h->st);
     delete h;
@@ -2310,6 +2393,7 @@ void daw_destroy(daw_handle* h) {
   if (h->ev1) cudaEventDestroy(h->ev1);
   if (h->d_err) cudaFree(h->d_err);
   if (h->d_qctr) cudaFree(h->d_qctr);
+  if (h->d_weights) cudaFree(h->d_weights);
   cudaStreamDestroy(h->st);
   delete h;
 }
@@ -2482,7 +2566,10 @@ void set_model(daw_handle* h, const float* vp, const float* rho, int32_t n1, int
     h->g = g;
     h->md = m;
     h->has_model = true;
-    if (h->ndatum > 0) h->datum = make_stations(h, h->model_pool, "datum", h->datum_tab.data(), h->ndatum);
+    if (h->ndatum > 0) {
+      h->datum = make_stations(h, h->model_pool, "datum", h->datum_tab.data(), h->ndatum);
+      sync(h);
+    }
 }
 
 }  // namespace
@@ -2504,6 +2591,7 @@ int daw_set_datum(daw_handle* h, const int32_t* tab, int32_t n) {
     h->datum_tab.assign(tab, tab + (size_t)n * 5);
     h->ndatum = n;
     h->datum = make_stations(h, h->model_pool, "datum", tab, n);
+    sync(h);  // `tab` has been read
     drop_graphs(h);
   });
 }
@@ -2519,8 +2607,8 @@ int daw_submodeling(daw_handle* h, const float* s, int32_t nt, const int32_t* is
     c.type_src = type_src;
     check_table(h, is5, 1, true, "is");
     std::memcpy(c.src5, is5, sizeof c.src5);
-    c.src = make_stations(h, h->pool, "shot0.src", is5, 1);
-    c.srcmap = make_map(h, h->pool, "shot0.srcmap", is5, 1, &c.srcinfo);
+    c.src = make_stations(h, h->pool, "shot0.src", c.src5, 1);
+    c.srcmap = make_map(h, h->pool, "shot0.srcmap", c.src5, 1, c.src, &c.srcinfo);
     upload(c.d_s, s, (size_t)nt * 4, h->st);
     Batch b;
     b.shots.push_back(&c);

@@ -97,6 +97,8 @@ void hicks_tile(int ia1, int ia2, int nfs, float* tile) {
   }
 }
 
+const float* hicks_weights() { return &weights().w[0][0]; }
+
 void hicks_locate(float z, float x, float h, int ofs, int32_t out[5]) {
   const float pos[2] = {z, x};
   for (int d = 0; d < 2; ++d) {

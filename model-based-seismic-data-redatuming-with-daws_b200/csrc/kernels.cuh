@@ -117,6 +117,12 @@ void hicks_gather(const StationsDev& st, const float* origin, int ld, int shift,
                   int hi2, float* out, int out_stride, int row, int nrows,
                   size_t field_stride, cudaStream_t s);
 
+// Station tables on the device (tables.cu): ix1, ix2 and the tiles of the n
+// stations of a (n,5) table, and the entries of an injection map with m slots a
+// point (col_lo, col_hi, col_base are set).
+void station_tiles(const int* tab, int n, const float* weights, const StationsDev& s, cudaStream_t st);
+void injection_map(const StationsDev& s, int n2e, int m, const InjMapDev& map, cudaStream_t st);
+
 // ---------------------------------------------------------------------------
 // MINRES vector kernels (minres.cu)
 // ---------------------------------------------------------------------------
