@@ -528,37 +528,74 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Sum of 0.5*sp^2 over a stage-A history (the esource `cost`).
-template <bool FP16>
-__global__ void k_hist_cost(const void* hist, const unsigned* amax, int nt, int n1, int n2,
-                            int inner_ld, int inner_off, size_t field_stride, double* out) {
-  __shared__ double sh[256];
-  double acc = 0;
-  const size_t per = (size_t)n1 * n2;
-  const size_t total = per * nt;
-  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total;
-       q += (size_t)gridDim.x * blockDim.x) {
-    const int it = (int)(q / per);
-    const size_t r = q % per;
-    const int i1 = (int)(r % n1), i2 = (int)(r / n1);
-    const size_t o = (size_t)it * 3 * field_stride + inner_off + i1 + (size_t)inner_ld * i2;
-    float v;
-    if (FP16) {
-      unsigned b = 0;
-      for (int s = 0; s < kAmaxSlots; ++s) b = max(b, amax[(size_t)it * 3 * kAmaxSlots + s]);
-      v = __half2float(static_cast<const __half*>(hist)[o]) * pow2f(amax_exponent(b) - 15);
-    } else {
-      v = static_cast<const float*>(hist)[o];
+// Sum of 0.5*sp^2 over a stage-A history (the esource `cost`).  A block takes
+// (step, 16 columns) tasks and reads V values a load; the step's scale is looked
+// up once a task and applied to its sum (a power of two: exact).  The squares of
+// FP16 values are exact in FP32; everything else is FP64.
+// Bound by reading the field once.  Measured on 751 x 2301 (1590 steps in three
+// shots, 5.5 GB): 2 ms against 17 ms for a thread per value that looked up the
+// 32 scale slots and divided its index down for each.
+constexpr int kCostCols = 16;
+template <bool FP16, int V>
+__global__ void __launch_bounds__(256)
+    k_hist_cost(const void* hist, const unsigned* amax, int nt, int n1, int n2, int inner_ld,
+                int inner_off, size_t field_stride, double* out) {
+  __shared__ double sh[8];
+  const int lane = threadIdx.x & 31;
+  const int nv = (inner_ld + V - 1) / V;  // loads a column
+  const int chunks = (n2 + kCostCols - 1) / kCostCols;
+  double total = 0;
+  for (long long task = blockIdx.x; task < (long long)nt * chunks; task += gridDim.x) {
+    const int it = (int)(task / chunks), c0 = (int)(task - (long long)it * chunks) * kCostCols;
+    const int n = min(kCostCols, n2 - c0) * nv;
+    double acc = 0;
+#pragma unroll 2
+    for (int q = threadIdx.x; q < n; q += 256) {
+      const int c = q / nv, r = (q - c * nv) * V;
+      const size_t o = (size_t)it * 3 * field_stride + (size_t)inner_ld * (c0 + c) + r;
+      float v[V];
+      if (FP16) {
+        if constexpr (V == 8) {
+          const uint4 x = __ldcs(reinterpret_cast<const uint4*>(static_cast<const __half*>(hist) + o));
+          const unsigned w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+            v[2 * k] = f.x;
+            v[2 * k + 1] = f.y;
+          }
+        } else {
+          v[0] = __half2float(static_cast<const __half*>(hist)[o]);
+        }
+      } else {
+        if constexpr (V == 4) {
+          const float4 x = __ldcs(reinterpret_cast<const float4*>(static_cast<const float*>(hist) + o));
+          v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        } else {
+          v[0] = static_cast<const float*>(hist)[o];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const int i = r + k - inner_off;
+        if (i < 0 || i >= n1) continue;  // rows beside the physical ones are not written
+        acc += FP16 ? (double)(v[k] * v[k]) : (double)v[k] * (double)v[k];
+      }
     }
-    acc += 0.5 * (double)v * (double)v;
+    double scale = 0.5;
+    if (FP16) {
+      const int e = amax_exponent(__reduce_max_sync(0xffffffffu, amax[(size_t)it * 3 * kAmaxSlots + lane])) - 15;
+      scale = scalbn(0.5, 2 * e);
+    }
+    total += scale * acc;
   }
-  sh[threadIdx.x] = acc;
+  for (int s = 16; s > 0; s >>= 1) total += __shfl_down_sync(0xffffffffu, total, s);
+  if (lane == 0) sh[threadIdx.x >> 5] = total;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; ++k) total += sh[k];
+    atomicAdd(out, total);
   }
-  if (threadIdx.x == 0) atomicAdd(out, sh[0]);
 }
 
 int host_bps(const Grid& g, int np) {
@@ -632,13 +669,18 @@ void fused_v_step(const Grid& g, const ModelDev& m, const FusedLaunch& L, int mo
 void history_cost(const void* hist, int fp16, const unsigned* amax, int nt, int n1, int n2,
                   int inner_ld, int inner_off, size_t field_stride, double* out,
                   cudaStream_t st) {
-  const int blocks = 148 * 4;
+  const int blocks = 148 * 8;
+  // whole 16-byte loads where columns start at 16-byte boundaries: always in the
+  // fused kernels' layout, by chance in the plain kernels'
+  const int v = fp16 ? 8 : 4;
+  const bool wide = inner_ld % v == 0 && field_stride % v == 0;
+  auto run = [&](auto k) {
+    k<<<blocks, 256, 0, st>>>(hist, amax, nt, n1, n2, inner_ld, inner_off, field_stride, out);
+  };
   if (fp16)
-    k_hist_cost<true><<<blocks, 256, 0, st>>>(hist, amax, nt, n1, n2, inner_ld, inner_off,
-                                              field_stride, out);
+    wide ? run(k_hist_cost<true, 8>) : run(k_hist_cost<true, 1>);
   else
-    k_hist_cost<false><<<blocks, 256, 0, st>>>(hist, amax, nt, n1, n2, inner_ld, inner_off,
-                                               field_stride, out);
+    wide ? run(k_hist_cost<false, 4>) : run(k_hist_cost<false, 1>);
 }
 
 }  // namespace daw
