@@ -206,7 +206,11 @@ __device__ __forceinline__ unsigned group_max(const u64* s, int G, unsigned tag,
 // Two maxima over the group's CTAs, by the extra warps: every CTA has stored
 // its tagged words at s and s + stride; the leader collects them and stores the
 // results to each CTA's own line at r.  (All CTAs polling all words made the lines
-// they share the bottleneck: 3 us an exchange with 126 CTAs.)
+// they share the bottleneck: 3 us an exchange with 126 CTAs.  Each CTA storing its
+// words to an array of every other, 20000 scattered stores, cost 1.4 us more a step
+// at 151 x 461.  Exchanges with a whole step of time, the histories stored a step
+// later from a copy: no gain, 3.6 against 3.7 us there and 4.6 against 4.2 at
+// 301 x 703.)
 constexpr int kLine = 16;  // words of a 128-byte line
 __device__ __forceinline__ uint2 exchange_max(const u64* s, size_t stride, int fields, u64* r, int b,
                                               int G, int leader, unsigned tag, Poll& w) {
@@ -399,7 +403,7 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, i
   l.term = take(pts * m * 4);
   l.tsta = take(pts * m * 2);
   l.tkap = take(pts * 4);
-  l.amp = take((nsta + 1) * 4);
+  l.amp = take(2 * (nsta + 1) * 4);  // amplitudes of one step and the next
   l.stage = take(quads * C * 16);    // pressure of the gather rectangles [quad][column]
   l.misc = take(64 * 4 + 16);
   l.total = o;
@@ -425,12 +429,12 @@ __host__ __device__ inline int aux_warp(int RB, int CG) {
 }
 
 // The injection terms ((c dt) amp) kappa of one step, by thread t of nt.
-__device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int pts, int m, int t, int nt) {
+__device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int pts, int m, const float* amp,
+                                          int t, int nt) {
   const float2* cd = reinterpret_cast<const float2*>(sm + l.tcd);
   float2* term = reinterpret_cast<float2*>(sm + l.term);
   const ushort2* sta = reinterpret_cast<const ushort2*>(sm + l.tsta);
   const float* kap = reinterpret_cast<const float*>(sm + l.tkap);
-  const float* amp = reinterpret_cast<const float*>(sm + l.amp);
   const int mh = m / 2;
   for (int p = t; p < pts; p += nt) {
     const float kv = kap[p];
@@ -483,7 +487,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   Q4* const ROW = reinterpret_cast<Q4*>(sm + l.row) + rb * 32 + lane;
   const int NP = RB * 32;
   float* const TERM = reinterpret_cast<float*>(sm + l.term);
-  float* const AMP = reinterpret_cast<float*>(sm + l.amp);
+  auto amp = [&](int it) { return reinterpret_cast<float*>(sm + l.amp) + (it & 1) * (L.inj_sta + 1); };
   unsigned* const WM = reinterpret_cast<unsigned*>(sm + l.misc);     // [3] maxima: p, vx, vz
   float* const SC = reinterpret_cast<float*>(sm + l.misc + 16 * 4);  // scales
   unsigned* const TB = reinterpret_cast<unsigned*>(sm + l.misc + 64 * 4);
@@ -603,13 +607,25 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       for (int k = tid; k < ipts; k += blockDim.x)  // rows above the surface: px stays zero
         tk[k] = ih.x + k % ih.y < fsrows ? 0.f : S.inj.kap[o + k];
       for (int k = tid; k <= ih.w; k += blockDim.x)
-        AMP[k] = k < ih.w ? S.amp[(size_t)(first - 1) * S.nsta + ih.z + k] : 0.f;
+        amp(first - 1)[k] = k < ih.w ? S.amp[(size_t)(first - 1) * S.nsta + ih.z + k] : 0.f;
+      if (tid == 0) amp(first)[ih.w] = 0.f;
     }
   }
   __syncthreads();
+  // Amplitudes of step it + 1 to amp(it), by the extra warp: a step ahead and
+  // without waiting, since they come from memory and the warp's exchange follows
+  // (stage A at 151 x 461: 3.7 us a step against 3.9 with the loads waited for).
+  auto fetch_amp = [&](int it) {
+    if (!kB && ipts > 0 && it < last)
+      for (int k = lane; k < ih.w; k += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(amp(it) + k)),
+                     "l"(S.amp + (size_t)it * S.nsta + ih.z + k)
+                     : "memory");
+  };
+  if (aux) fetch_amp(first);
   // the warps but the extra one
   const int it0 = tid - (warp > aux_warp(RB, L.CG) ? 32 : 0), itn = blockDim.x - 32;
-  if (ipts > 0 && !aux) inj_terms(sm, l, ipts, im, it0, itn);
+  if (ipts > 0 && !aux) inj_terms(sm, l, ipts, im, amp(first - 1), it0, itn);
 
   const u64 nz = L.nz;
   auto mul2 = [&](u64 x, u64 y) { return fma2(x, y, nz); };
@@ -740,6 +756,30 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   auto results = [&](int phase, int s) {
     return L.slots + (size_t)8 * gridDim.x +
            ((size_t)(phase * 2 + (s & 1)) * gridDim.x + grp * G) * kLine;
+  };
+  auto words = [&](int phase, int s) {
+    return L.slots + (size_t)(phase * 4 + (s & 1) * 2) * gridDim.x + grp * G;
+  };
+  // of step s: maxima to memory, scales to SC
+  auto exchange_p = [&](int s) {
+    const uint2 m = exchange_max(words(0, s), 0, 1, results(0, s), b, G, 0, L.tag0 + (unsigned)s, poll);
+    if (lane == 0) {
+      SC[0] = pow2f(15 - amax_exponent(m.x));
+      if (b == 0) S.amax[(size_t)(s - 1) * 3 * kAmaxSlots] = m.x;
+    }
+  };
+  auto exchange_v = [&](int s) {
+    const uint2 m = exchange_max(words(1, s), gridDim.x, 2, results(1, s), b, G, vleader,
+                                 L.tag0 + (unsigned)s, poll);
+    if (lane == 0) {
+      SC[1] = pow2f(15 - amax_exponent(m.x));
+      SC[2] = pow2f(15 - amax_exponent(m.y));
+      if (b == 0) {
+        unsigned* am = S.amax + (size_t)(s - 1) * 3 * kAmaxSlots;
+        am[kAmaxSlots] = m.x;
+        am[2 * kAmaxSlots] = m.y;
+      }
+    }
   };
   sync_cta();
 
@@ -932,24 +972,11 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         }
       }
     } else if (aux) {
-      if (kA && it > first) {            // velocity maxima of the previous step
-        if (FP16) {
-          const uint2 m = exchange_max(L.slots + (size_t)(4 + ((it - 1) & 1) * 2) * gridDim.x + grp * G,
-                                       gridDim.x, 2, results(1, it - 1), b, G, vleader, tag - 1, poll);
-          const unsigned vx = m.x, vz = m.y;
-          if (lane == 0) {
-            SC[1] = pow2f(15 - amax_exponent(vx));
-            SC[2] = pow2f(15 - amax_exponent(vz));
-            if (b == 0) {
-              unsigned* am = S.amax + (size_t)(it - 2) * 3 * kAmaxSlots;
-              am[kAmaxSlots] = vx;
-              am[2 * kAmaxSlots] = vz;
-            }
-          }
-        }
+      if (kA && FP16 && it > first) exchange_v(it - 1);  // velocity maxima of the previous step
+      if (!kB) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        fetch_amp(it + 1);
       }
-      if (!kB && ipts > 0 && it < last)  // amplitudes of the next step
-        for (int k = lane; k < ih.w; k += 32) AMP[k] = S.amp[(size_t)it * S.nsta + ih.z + k];
       if (kB) prefetch_b(it + 2);
     }
     if (extra) {
@@ -958,7 +985,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
     }
     sync_cta();
     // =============== velocity half step ===============
-    if (!kB && ipts > 0 && it < last && !aux) inj_terms(sm, l, ipts, im, it0, itn);
+    if (!kB && ipts > 0 && it < last && !aux) inj_terms(sm, l, ipts, im, amp(it), it0, itn);
     if (comp) {
       const Q4 d1b = lds4(ROW + 2 * NP), bw1 = lds4(ROW + 3 * NP);
       const u64 INVX = splat(kA && FP16 ? SC[1] : 1.f), INVZ = splat(kA && FP16 ? SC[2] : 1.f);
@@ -1147,13 +1174,8 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           if (m >= 0x7f800000u) atomicOr(L.err, kErrNonFinite);
         }
         if (FP16) {
-          u64* sl = L.slots + (size_t)((it & 1) * 2) * gridDim.x + grp * G;
-          if (lane == 0) word_store(sl + b, (u64)tag << 32 | m);
-          const unsigned p = exchange_max(sl, 0, 1, results(0, it), b, G, 0, tag, poll).x;
-          if (lane == 0) {
-            SC[0] = pow2f(15 - amax_exponent(p));
-            if (b == 0) S.amax[(size_t)(it - 1) * 3 * kAmaxSlots] = p;
-          }
+          if (lane == 0) word_store(words(0, it) + b, (u64)tag << 32 | m);
+          exchange_p(it);
         }
       }
       if (staged) {
@@ -1181,9 +1203,8 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         WM[1] = WM[2] = 0;
         if (max(x, z) >= 0x7f800000u) atomicOr(L.err, kErrNonFinite);
         if (FP16) {
-          u64* sl = L.slots + (size_t)(4 + (it & 1) * 2) * gridDim.x + grp * G;
-          word_store(sl + b, (u64)tag << 32 | x);
-          word_store(sl + gridDim.x + b, (u64)tag << 32 | z);
+          word_store(words(1, it) + b, (u64)tag << 32 | x);
+          word_store(words(1, it) + gridDim.x + b, (u64)tag << 32 | z);
         }
       }
       __syncwarp();
@@ -1192,21 +1213,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
 
   // ---- the last step's histories
   if (kA) {
-    if (aux && FP16) {
-      const unsigned tag = L.tag0 + (unsigned)last;
-      const uint2 m = exchange_max(L.slots + (size_t)(4 + (last & 1) * 2) * gridDim.x + grp * G,
-                                   gridDim.x, 2, results(1, last), b, G, vleader, tag, poll);
-      const unsigned vx = m.x, vz = m.y;
-      if (lane == 0) {
-        SC[1] = pow2f(15 - amax_exponent(vx));
-        SC[2] = pow2f(15 - amax_exponent(vz));
-        if (b == 0) {
-          unsigned* am = S.amax + (size_t)(last - 1) * 3 * kAmaxSlots;
-          am[kAmaxSlots] = vx;
-          am[2 * kAmaxSlots] = vz;
-        }
-      }
-    }
+    if (aux && FP16) exchange_v(last);
     __syncthreads();
   }
   if (comp && (kA || L.save)) {
