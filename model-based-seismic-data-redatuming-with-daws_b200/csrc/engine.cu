@@ -1132,6 +1132,75 @@ void make_tables(daw_handle* h, const ShotCtx& c, const MapInfo& info, const Inj
   t->dev = d;
 }
 
+// A pool buffer whose words start at zero (no step tag is zero).
+void* zeroed(daw_handle* h, const std::string& name, size_t bytes) {
+  const bool fresh = h->pool.bufs[name].bytes < bytes;
+  void* p = h->pool.get(name, bytes);
+  if (fresh) CK(cudaMemsetAsync(p, 0, bytes, h->st));
+  return p;
+}
+
+// Shape of a batch's runs of `mode` on chip: the tables and stages are sized for
+// the largest of its shots, active or not.
+struct ResidentShape {
+  int G = 0, RB = 0, pts = 0, m = 0, nsta = 0, quads = 0, occ = 0;
+  int room = 0;  // shots whose CTAs are resident together
+};
+ResidentShape resident_shape(daw_handle* h, const Batch& b, int mode) {
+  ResidentShape s;
+  s.G = (h->g.n2e + b.res_cols - 1) / b.res_cols;
+  s.RB = (h->g.n1e + 127) / 128;
+  bool stage = true;  // staged only when every shot's rectangles are
+  for (const ShotCtx* c : b.shots) {
+    if (mode == FM_FWD || mode == FM_STAGE_A) {
+      const ResidentInj& t = mode == FM_FWD ? c->srctab.dev : c->rectab.dev;
+      s.pts = std::max(s.pts, t.pts);
+      s.m = std::max(s.m, t.m);
+      s.nsta = std::max(s.nsta, t.nsta);
+    }
+    Box box[2];
+    gather_boxes(h, b, *c, mode, box);
+    const int q = staged_quads(b.res_cols, box);
+    stage = stage && (q > 0 || box[0].elems() + box[1].elems() == 0);
+    s.quads = std::max(s.quads, q);
+  }
+  if (!stage) s.quads = 0;
+  s.occ = resident_occupancy(mode == FM_STAGE_B_ES ? FM_STAGE_B : mode, h->opt.history_fp16 != 0,
+                             h->md.rbw1 != nullptr, b.res_cols, s.RB,
+                             resident_smem(b.res_cols, s.RB, s.pts, s.m, s.nsta, s.quads));
+  s.room = s.occ * h->sms / s.G;
+  return s;
+}
+
+// Buffers of a batch's runs of `mode` on chip, for as many shots as run
+// together: halo words, maxima, and the rectangle buffer, which takes less (the
+// loops then run in shorter launches) where memory is short of its usual size.
+// Throws DAW_ERR_OOM when one step of the rectangles does not fit either.
+void reserve_resident(daw_handle* h, const Batch& b, int mode) {
+  const ResidentShape s = resident_shape(h, b, mode);
+  const size_t q = std::max(1, std::min({s.room, kResShots, (int)b.shots.size()}));
+  zeroed(h, "resident.halo", 4 * q * s.G * 3 * s.RB * 64 * sizeof(ulonglong2));
+  zeroed(h, "resident.slots", 72 * q * s.G * sizeof(unsigned long long));
+  std::vector<size_t> elems;
+  for (const ShotCtx* c : b.shots) {
+    Box box[2];
+    gather_boxes(h, b, *c, mode, box);
+    elems.push_back(box[0].elems() + box[1].elems());
+  }
+  std::sort(elems.rbegin(), elems.rend());
+  size_t one = 0;  // the largest group's step
+  for (size_t i = 0; i < q; ++i) one += elems[i] * sizeof(float);
+  if (!one) return;
+  for (size_t bytes = std::max(one, std::min(kRectBytes, one * b.max_nt));; bytes = std::max(one, bytes / 2)) {
+    try {
+      h->pool.get("resident.rect", bytes);
+      return;
+    } catch (const DawError& e) {
+      if (e.code != DAW_ERR_OOM || bytes == one) throw;
+    }
+  }
+}
+
 // Decides and prepares the on-chip path for a batch's runs of `modes`; false:
 // the batch runs from global memory.
 bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
@@ -1144,20 +1213,16 @@ bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
         if (mode == FM_FWD) make_tables(h, *c, c->srcinfo, c->srcmap, b.res_cols, "srctab", &c->srctab);
         if (mode == FM_STAGE_A) make_tables(h, *c, c->recinfo, c->recmap, b.res_cols, "rectab", &c->rectab);
       }
+    for (int mode : modes) {
+      if (resident_shape(h, b, mode).room < 1) return false;
+      reserve_resident(h, b, mode);
+    }
   } catch (const DawError& e) {
     if (e.code != DAW_ERR_OOM) throw;
     return false;
   }
   b.resident = true;
   return true;
-}
-
-// A pool buffer whose words start at zero (no step tag is zero).
-void* zeroed(daw_handle* h, const std::string& name, size_t bytes) {
-  const bool fresh = h->pool.bufs[name].bytes < bytes;
-  void* p = h->pool.get(name, bytes);
-  if (fresh) CK(cudaMemsetAsync(p, 0, bytes, h->st));
-  return p;
 }
 
 // The time loops of `mode` on chip: the active shots in groups that share a
@@ -1182,38 +1247,19 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
   auto inj_of = [&](const ShotCtx& c) {
     return mode == FM_FWD ? c.srctab.dev : mode == FM_STAGE_A ? c.rectab.dev : ResidentInj{};
   };
-  for (const ShotCtx* c : act) {
-    const ResidentInj t = inj_of(*c);
-    L.inj_pts = std::max(L.inj_pts, t.pts);
-    L.inj_m = std::max(L.inj_m, t.m);
-    L.inj_sta = std::max(L.inj_sta, t.nsta);
-  }
-  // staged only when every shot's rectangles are
-  bool stage = true;
-  for (const ShotCtx* c : act) {
-    Box box[2];
-    gather_boxes(h, b, *c, mode, box);
-    const int q = staged_quads(L.C, box);
-    stage = stage && (q > 0 || box[0].elems() + box[1].elems() == 0);
-    L.quads = std::max(L.quads, q);
-  }
-  if (!stage) L.quads = 0;
-  const int occ = resident_occupancy(
-      kmode, fp16, h->md.rbw1 != nullptr, L.C, L.RB,
-      resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads));
-  const int room = occ * h->sms / L.G;  // shots whose CTAs are resident together
-  if (room < 1) throw DawError{DAW_ERR_STATE, "on-chip time loop does not fit"};
-  const int q = std::min({room, kResShots, (int)act.size()});
+  const ResidentShape shape = resident_shape(h, b, mode);
+  L.inj_pts = shape.pts;
+  L.inj_m = shape.m;
+  L.inj_sta = shape.nsta;
+  L.quads = shape.quads;
+  const int q = std::min({shape.room, kResShots, (int)act.size()});
   h->tim.kernel_family[mode] = 2;
   h->tim.tile_cols[mode] = L.C;
-  h->tim.ctas_per_sm[mode] = occ;
+  h->tim.ctas_per_sm[mode] = shape.occ;
   h->tim.ctas_per_sm_v[mode] = 0;
   h->tim.shots_per_launch[mode] = q;
-  const size_t ctas = (size_t)L.G * q;
-  L.halo = static_cast<ulonglong2*>(
-      zeroed(h, "resident.halo", 4 * ctas * 3 * L.RB * 64 * sizeof(ulonglong2)));
-  L.slots = static_cast<unsigned long long*>(
-      zeroed(h, "resident.slots", 72 * ctas * sizeof(unsigned long long)));
+  L.halo = h->pool.get_t<ulonglong2>("resident.halo", 0);
+  L.slots = h->pool.get_t<unsigned long long>("resident.slots", 0);
   for (size_t g0 = 0; g0 < act.size(); g0 += q) {
     const int n = (int)std::min<size_t>(q, act.size() - g0);
     L.groups = n;
@@ -1235,10 +1281,9 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
     int chunk = nsteps;
     float* rect = nullptr;
     if (rect_elems) {
-      size_t bytes = std::min<size_t>(kRectBytes, rect_elems * sizeof(float) * nsteps);
-      bytes = std::max(bytes, rect_elems * sizeof(float));
-      rect = static_cast<float*>(h->pool.get("resident.rect", bytes));
-      chunk = (int)std::min<size_t>(nsteps, bytes / (rect_elems * sizeof(float)));
+      const DevBuf& buf = h->pool.bufs["resident.rect"];
+      rect = static_cast<float*>(buf.p);
+      chunk = (int)std::min<size_t>(nsteps, buf.bytes / (rect_elems * sizeof(float)));
       // launches of similar length
       chunk = (nsteps + (nsteps + chunk - 1) / chunk - 1) / ((nsteps + chunk - 1) / chunk);
     }

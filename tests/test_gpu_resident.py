@@ -115,6 +115,27 @@ def test_long_loop_is_cut_into_launches(pkg):
         assert np.array_equal(x, y)
 
 
+def test_little_device_memory(pkg):
+    """With a quarter GB of device memory left the kept rectangles get a smaller
+    buffer and the loop more launches."""
+    import torch
+    c = workload(pkg, 380, 1201, 13, 700, 9, rows=(2.0, 360.0))
+    with handle(pkg, c) as h:
+        ref = h.submodeling(c["s"], c["src"], c["rec"])[0]
+        launches = h.timing()["kernel_launches"]
+    with handle(pkg, c) as h:
+        free, _ = torch.cuda.mem_get_info()
+        held = torch.empty(free - (256 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            got = h.submodeling(c["s"], c["src"], c["rec"])[0]
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        tim = h.timing()
+    assert tim["kernel_family"][0] == RESIDENT and tim["kernel_launches"] > launches
+    assert np.array_equal(got, ref)
+
+
 def test_uneven_batch_equals_split_kernels(pkg):
     """Shots of different lengths and spreads share launches."""
     base = workload(pkg, 90, 160, 14, 160, 19)
