@@ -688,6 +688,7 @@ struct Batch {
   bool no_datum = false;  // forward-only batches: no datum gathers
   bool resident = false;  // the run's time loops stay on chip (resident.cuh)
   int res_cols = 0;       // with that many columns per CTA
+  bool step = false;      // one kernel per step, chosen by the grid's size
   int slot0 = 0;
 };
 
@@ -703,8 +704,8 @@ int chunk_of(const daw_handle* h) { return h->opt.chunk; }
 // one-kernel-per-step family is pinned, the step kernels' unless the split
 // family is pinned (DAW_OPT_STEP_KERNEL 0 / 1; 2 = autotuned needs both).
 bool tma_path(const daw_handle* h) { return h->opt.fused && h->opt.chunk == 0; }
-bool split_maps(const daw_handle* h) { return tma_path(h) && h->opt.step != 1; }
-bool step_maps(const daw_handle* h) { return tma_path(h) && h->opt.step != 0; }
+bool split_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && h->opt.step != 1 && !b.step; }
+bool step_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && (h->opt.step != 0 || b.step); }
 // Family of the windows of a checkpointed shot (not tuned): the step kernels
 // only when pinned.
 bool windowed_step(const daw_handle* h) { return tma_path(h) && h->opt.step == 1; }
@@ -754,7 +755,7 @@ void fill_shot_devices(daw_handle* h, Batch& b, int mode, const Window* w = null
     }
   }
   upload(b.d_shots, b.h_shots.data(), b.h_shots.size() * sizeof(ShotDevice), h->st);
-  if (step_maps(h)) {
+  if (step_maps(h, b)) {
     // tensor maps of every shot for both tile widths: [tile width 16 | 32][shot]
     const size_t n = b.shots.size();
     std::vector<StepMaps> maps(2 * n);
@@ -772,7 +773,7 @@ void fill_shot_devices(daw_handle* h, Batch& b, int mode, const Window* w = null
     upload(b.d_smaps, maps.data(), maps.size() * sizeof(StepMaps), h->st);
     sync(h);  // `maps` goes out of scope
   }
-  if (split_maps(h)) {
+  if (split_maps(h, b)) {
     // tensor maps of every shot's fields (the TMA kernels' operands)
     std::vector<TmaMaps> maps(b.shots.size());
     for (size_t i = 0; i < b.shots.size(); ++i) {
@@ -869,14 +870,15 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
     if (b.shots[i]->active) act.push_back((int)i);
   const int nact = std::max<int>(1, (int)act.size());
   const daw_handle::Tuned split_default{0, 32, occ_p, occ_v, 0, 0.f};
-  if (!may_time) {  // checkpointed windows: the named family, default shapes
-    if (h->opt.step == 1) {
-      const int tc = h->opt.tile_cols ? h->opt.tile_cols : 32;
-      const int occ = std::max(1, std::min(h->step_occ[tmode][f][tc == 32 ? 1 : 0], 3));
-      return {1, tc, h->opt.ctas_per_sm ? std::min(h->opt.ctas_per_sm, occ) : occ, 0, 0, 0.f};
-    }
-    return split_default;
+  // Not tuned: checkpointed windows, which take the named family, and large grids,
+  // where tiles of 32 columns and as many CTAs as fit are the fastest choice or
+  // within 1 % of it in every mode (150 MB to 1 GB of state and both histories).
+  if (b.step || (!may_time && h->opt.step == 1)) {
+    const int tc = h->opt.tile_cols ? h->opt.tile_cols : 32;
+    const int occ = std::max(1, std::min(h->step_occ[tmode][f][tc == 32 ? 1 : 0], 3));
+    return {1, tc, h->opt.ctas_per_sm ? std::min(h->opt.ctas_per_sm, occ) : occ, 0, 0, 0.f};
   }
+  if (!may_time) return split_default;
   char key[192];
   std::snprintf(key, sizeof key, "m%d.f%d.g%dx%d.p%d.s%d.a%d.r%d.d%d.k%d.t%d.c%d.rho%d", tmode,
                 f, h->g.n1, h->g.n2, h->g.npml, L.nshots, nact, L.max_rec, L.max_datum,
@@ -928,7 +930,7 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
     timed = true;
     if (cd.us_per_step < best.us_per_step) best = cd;
   };
-  if (h->opt.step != 1) {
+  if (h->opt.step != 1 && !b.step) {
     // shots per launch (default shapes), then the CTAs per SM for the best
     std::vector<int> ks;
     for (int k : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
@@ -942,7 +944,7 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
         for (int vc = 1; vc <= occ_v; ++vc)
           if (!(timed && pc == occ_p && vc == occ_v)) consider({0, 32, pc, vc, kbest, 0.f});
   }
-  if (h->opt.step != 0 && !h->md.rbw1)  // the step family has no density variant
+  if ((h->opt.step != 0 || b.step) && !h->md.rbw1)  // the step family has no density variant
     for (int tc : {16, 32}) {
       if (h->opt.tile_cols && h->opt.tile_cols != tc) continue;
       // a pinned CTA count above what fits is clamped to the occupancy
@@ -1201,10 +1203,30 @@ void reserve_resident(daw_handle* h, const Batch& b, int mode) {
   }
 }
 
+// From global memory, one kernel per step moves 36 bytes a point and step and two
+// kernels 52 of which part stays in L2: us per step of both (tuned, FP16 histories)
+//   points    forward        stage A        stage B
+//   2.9 M     38 against 33    37 against 36    40 against 33
+//   4.0 M     47 against 42    43 against 44    48 against 43
+//   4.9 M     52 against 54    50 against 53    53 against 53
+//   5.7 M     58 against 69    59 against 68    61 against 66
+//   10.7 M    93 against 112   97 against 126   103 against 114
+//   17.0 M    137 against 170  151 against 193  155 against 172
+//   20.3 M    158 against 190  176 against 223  184 against 201
+// Windowed histories keep to the split kernels, as with DAW_OPT_STEP_KERNEL = 2;
+// the one-kernel family has no density variant.
+constexpr size_t kStepElems = (size_t)5 << 20;
+bool large_grid(const daw_handle* h, const Batch& b) {
+  for (const ShotCtx* c : b.shots)
+    if (c->hist_win > 0) return false;
+  return resident_family(h) && !h->md.rbw1 && h->g.ext_elems() >= kStepElems;
+}
+
 // Decides and prepares the on-chip path for a batch's runs of `modes`; false:
 // the batch runs from global memory.
 bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
   b.resident = false;
+  b.step = large_grid(h, b);
   b.res_cols = resident_columns(h, b, modes);
   if (!b.res_cols) return false;
   try {
@@ -1222,6 +1244,7 @@ bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
     return false;
   }
   b.resident = true;
+  b.step = false;
   return true;
 }
 
