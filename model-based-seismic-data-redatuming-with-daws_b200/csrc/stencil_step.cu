@@ -1,5 +1,5 @@
 // One kernel per time step: the pressure update and the velocity update of
-// step `it` in a single pass over the grid (the default fused path).
+// step `it` in a single pass over the grid (the default on large grids).
 //
 // The reference's time step (src/submodeling2.f90:148-236 forward,
 // :1013-1087 stage A, :1104-1192 stage B) is a pressure update from the
@@ -47,7 +47,11 @@
 namespace daw {
 namespace {
 
-constexpr int kT = 256;          // threads per CTA (8 warps)
+// Warps per CTA.  Stage B's tiles of 32 columns have room for one CTA per SM (their
+// stages hold the histories too); with 16 warps instead of 8 a step takes 60.8, 102.8
+// and 155.3 us on grids of 5.7, 10.7 and 17.0 M points against 62.8, 103.9 and 158.3.
+template <int MODE, int TC>
+constexpr int kWarps = (MODE == FM_STAGE_B || MODE == FM_STAGE_B_ES) && TC == 32 ? 16 : 8;
 constexpr int SR = 64;           // rows per tile (32 lanes x 2)
 constexpr int SH = 4;            // row halo of the field boxes (aligned start r0 - 4)
 constexpr int SB = SR + 2 * SH;  // 72 rows per field box
@@ -62,7 +66,6 @@ __host__ __device__ constexpr int pad128(int x) { return (x + 127) / 128 * 128; 
 
 template <int TC>
 struct SG {
-  static constexpr int CPT = TC / 8;  // columns per warp
   static constexpr int NX = TC + 6;   // vx box: columns c0-3 .. c0+TC+2
   static constexpr int NP = TC + 3;   // vz, px, pz, kappa boxes: c0-1 .. c0+TC+1
   static constexpr int kVX = pad128(SB * NX * 4);
@@ -222,13 +225,14 @@ __device__ __forceinline__ float warp_gather_pxpz(float* prod, const int* ix1p, 
 }
 
 template <int MODE, bool FP16, int TC>
-__global__ void __launch_bounds__(kT, TC == 16 ? 3 : 2)
+__global__ void __launch_bounds__(32 * kWarps<MODE, TC>, kWarps<MODE, TC> == 16 ? 1 : TC == 16 ? 3 : 2)
     k_step(const Grid g, const ModelDev m, const FusedLaunch L, const int it) {
   using G = SG<TC>;
   using H = Hist<FP16>;
   constexpr bool kB = G::stage_b(MODE);
   constexpr int kStage = G::stage(MODE, FP16);
-  constexpr int CPT = G::CPT, NP = G::NP;
+  constexpr int kT = 32 * kWarps<MODE, TC>, NP = G::NP;
+  constexpr int CPT = 32 * TC / kT;  // columns per warp
   constexpr bool kInj = (MODE == FM_FWD || MODE == FM_STAGE_A);
   extern __shared__ __align__(128) unsigned char smem[];
   float* amp_s = reinterpret_cast<float*>(smem + 2 * kStage);
@@ -439,7 +443,7 @@ __global__ void __launch_bounds__(kT, TC == 16 ? 3 : 2)
     do {  // the item; `break` ends it
     if (id.kind == 1) {
       // ---- gather unit: receivers / datum of step it - 1 from the input set
-      if (ss.defer && MODE != FM_STAGE_A) {
+      if (ss.defer && MODE != FM_STAGE_A && warp < 8) {
         float* prod = reinterpret_cast<float*>(smem) + warp * kGatherStride;
         const int sta = id.unit * 8 + warp;
         const float* opx = fld(sd, pin, 0);
@@ -943,7 +947,7 @@ __global__ void __launch_bounds__(kT, TC == 16 ? 3 : 2)
 template <int MODE, bool FP16, int TC>
 void launch_t(const Grid& g, const ModelDev& m, const FusedLaunch& L, int it, int grid,
               cudaStream_t st) {
-  launch_pdl(k_step<MODE, FP16, TC>, grid, kT, SG<TC>::smem(MODE, FP16), st, L.pdl != 0, g, m, L,
+  launch_pdl(k_step<MODE, FP16, TC>, grid, 32 * kWarps<MODE, TC>, SG<TC>::smem(MODE, FP16), st, L.pdl != 0, g, m, L,
              it);
 }
 
@@ -972,7 +976,7 @@ int occ_t() {
                            (int)sm) != cudaSuccess)
     return 0;
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_step<MODE, FP16, TC>, kT, sm) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_step<MODE, FP16, TC>, 32 * kWarps<MODE, TC>, sm) !=
       cudaSuccess)
     return 0;
   return n;
