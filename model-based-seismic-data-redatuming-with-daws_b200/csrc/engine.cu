@@ -707,8 +707,8 @@ bool tma_path(const daw_handle* h) { return h->opt.fused && h->opt.chunk == 0; }
 bool split_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && h->opt.step != 1 && !b.step; }
 bool step_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && (h->opt.step != 0 || b.step); }
 // Family of the windows of a checkpointed shot (not tuned): the step kernels
-// only when pinned.
-bool windowed_step(const daw_handle* h) { return tma_path(h) && h->opt.step == 1; }
+// when pinned or chosen by the grid's size.
+bool windowed_step(const daw_handle* h, const Batch& b) { return tma_path(h) && (h->opt.step == 1 || b.step); }
 
 // Device descriptors (and tensor maps) of the batch's shots for `mode`.  With
 // a window, stage A sees the window as a record of w->len steps whose
@@ -1213,12 +1213,9 @@ void reserve_resident(daw_handle* h, const Batch& b, int mode) {
 //   10.7 M    93 against 112   97 against 126   103 against 114
 //   17.0 M    137 against 170  151 against 193  155 against 172
 //   20.3 M    158 against 190  176 against 223  184 against 201
-// Windowed histories keep to the split kernels, as with DAW_OPT_STEP_KERNEL = 2;
-// the one-kernel family has no density variant.
+// The one-kernel family has no density variant.
 constexpr size_t kStepElems = (size_t)5 << 20;
-bool large_grid(const daw_handle* h, const Batch& b) {
-  for (const ShotCtx* c : b.shots)
-    if (c->hist_win > 0) return false;
+bool large_grid(const daw_handle* h) {
   return resident_family(h) && !h->md.rbw1 && h->g.ext_elems() >= kStepElems;
 }
 
@@ -1226,7 +1223,7 @@ bool large_grid(const daw_handle* h, const Batch& b) {
 // the batch runs from global memory.
 bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
   b.resident = false;
-  b.step = large_grid(h, b);
+  b.step = large_grid(h);
   b.res_cols = resident_columns(h, b, modes);
   if (!b.res_cols) return false;
   try {
@@ -1619,7 +1616,7 @@ void shot_operator_windowed(daw_handle* h, Batch& b, bool esource) {
   const size_t ne = h->g.ext_elems();
   // a saved state: the four fields of the current set (one-kernel-per-step
   // path) or px, pz, vx, vz, p (split kernels); ckpt slots hold 5 fields
-  const bool step = windowed_step(h);
+  const bool step = windowed_step(h, b);
   const size_t save_bytes = (step ? 4 : 5) * ne * sizeof(float);
   const int K = c.hist_win, nwin = (c.nt + K - 1) / K;
   float* const st_a = c.state;  // the slot's state block
