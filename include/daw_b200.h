@@ -76,15 +76,16 @@ enum daw_option {
                                 keeps whole histories. */,
   DAW_OPT_STEP_KERNEL = 9,   /* TMA kernel family (DAW_OPT_CHUNK = 0): 0 (default) =
                                 the time loop on chip where the grid fits the SMs'
-                                registers, shared and tensor memory, else (and with
-                                DAW_OPT_PDL) separate pressure and velocity kernels,
-                                shots per launch and CTAs per SM chosen by the
+                                registers, shared and tensor memory, else from 5 Mi
+                                padded points on one kernel per time step, else (and
+                                with DAW_OPT_PDL) separate pressure and velocity
+                                kernels, shots per launch and CTAs per SM chosen by the
                                 autotuner; 1 = one kernel
                                 per time step (pressure recomputed on the velocity
                                 stencil's halo, two alternating state sets), tile width
-                                and CTAs per SM autotuned; 2 = the family autotuned too
-                                (the windows of a checkpointed shot use the separate
-                                kernels unless 1 is set) */
+                                and CTAs per SM autotuned; 2 = one or separate kernels,
+                                autotuned (the windows of a checkpointed shot then use
+                                the separate kernels) */
   DAW_OPT_TILE_COLS = 10,    /* one-kernel-per-step tiles: 16 or 32 columns of 64
                                 rows; 0 (default) = chosen by the autotuner */
   DAW_OPT_CTAS_PER_SM = 11,  /* one-kernel-per-step CTAs per SM (1..3; a value above

@@ -701,8 +701,8 @@ struct Window {
 // with that many columns per thread.
 int chunk_of(const daw_handle* h) { return h->opt.chunk; }
 // Tensor maps needed by the TMA kernels: the split kernels' unless the
-// one-kernel-per-step family is pinned, the step kernels' unless the split
-// family is pinned (DAW_OPT_STEP_KERNEL 0 / 1; 2 = autotuned needs both).
+// one-kernel-per-step family is pinned or chosen by the grid's size, the step
+// kernels' then and where the family is autotuned (DAW_OPT_STEP_KERNEL = 2).
 bool tma_path(const daw_handle* h) { return h->opt.fused && h->opt.chunk == 0; }
 bool split_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && h->opt.step != 1 && !b.step; }
 bool step_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && (h->opt.step != 0 || b.step); }
@@ -852,9 +852,9 @@ void stop_clock(daw_handle* h, SimClock& clk, Batch& b, int mode, const Window* 
 //     occupancy CTAs per SM of each kernel;
 //   - with DAW_OPT_STEP_KERNEL = 2 or 1, one kernel per step with 16- or
 //     32-column tiles and 1 .. occupancy CTAs per SM (whole batch).
-// Only runs that start from the zero state are tuned; the windows of a
-// checkpointed shot take the family DAW_OPT_STEP_KERNEL names with default
-// shapes.  The trials change only what the run itself then overwrites: the
+// Only runs that start from the zero state are tuned, and large grids not at
+// all (below); the windows of a checkpointed shot take the family
+// DAW_OPT_STEP_KERNEL names with default shapes.  The trials change only what the run itself then overwrites: the
 // state (zeroed again afterwards, and the stage-A max-|x| slots cleared), the
 // first history slots and the first rows of the outputs.  The final esource,
 // whose first step also accumulates into the wavefield output, tunes as stage

@@ -45,11 +45,13 @@
 // ones the exchange latency (about 0.5 us per half step).  Tried and slower: the fields in
 // registers with all columns unrolled (30 us a step against 14: instruction
 // cache), lanes of two rows (13.2-14.0 us against 9.2-12.5 then: the same number of
-// instructions per lane), a separate copy of the column code for the edges.
+// instructions per lane), a separate copy of the column code for the edges, the
+// neighbours' words waited for inside the edge column after what does not need
+// them (stage A 3.9 us against 3.7 at 151 x 461: registers spill).
 // Measured per shot step against the split kernels (B200, FP16 histories):
 // 751 x 2301 (17 columns a CTA) forward 7.1 us against 20.1, stage A 10.8
 // against 20.7-23.0, stage B 9.1 against 19.7-24.7; 151 x 461 (4 columns)
-// 2.4-4.0 us against 12-15.
+// 2.4-3.7 us against 12-15.
 #include "resident.cuh"
 #include "tma.cuh"
 
