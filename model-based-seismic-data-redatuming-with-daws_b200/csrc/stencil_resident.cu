@@ -803,13 +803,13 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       const bool rhalo = hasr && redge && it > first, lhalo = hasl && clo < 2 && it > first;
       const unsigned events = (1u << jx) | (rhalo ? 1u << (C - 1) : 0u);
       const unsigned outs = (hasr ? 1u << (C - 1) : 0u) | (hasl ? 3u : 0u);
-      HT he[HR] = {};  // histories of columns 0 and 1
+      HT he[HR] = {};  // histories of the warp's columns below 2
       auto fetch = [&]() {
         if (rhalo) halo_fetch<1>(SH + 128, hin + hcta + 2 * hcol, hcol);
         if (lhalo) halo_fetch<2>(SH, hin - hcta, hcol);
-        if (kB && ledge) {
-          he[0] = ldh(hp, 0, lsrc);
-          he[1] = ldh(hp, 1, lsrc);
+        if (kB && clo < 2) {
+          he[0] = ldh(hp, clo, lsrc);
+          he[1] = ldh(hp, clo + 1, lsrc);
         }
       };
       auto put_left = [&]() {
@@ -948,12 +948,12 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       };
       for (int j = pj0, je = chi;;) {
         if (j < 2) {
-          if (je <= 2) fetch();
+          if (chi <= 2) fetch();  // else fetched at column jx
           put_left();
         }
         columns(j, je);
-        if (clo > 0 || je <= 2) break;
-        j = 0;  // the left edge's columns
+        if (clo > 1 || je <= 2) break;
+        j = clo;  // the left edge's columns
         je = 2;
         if (kB) {
           hq[0] = he[0];
@@ -1138,7 +1138,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       };
       for (int j = vj0, je = chi;;) {
         if (j == 0) {
-          if (je <= 1) fetch();
+          if (jx == 31) fetch();  // else fetched at column jx
           put_left();
         }
         if (j == C - 1 && rhalo) {  // the last column is the warp's only one

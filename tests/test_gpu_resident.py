@@ -43,6 +43,9 @@ def handle(pkg, c, **opt):
 GRIDS = [(14, 18, 3, 90), (102, 64, 13, 120), (103, 65, 13, 120), (486, 75, 13, 80),
          (934, 60, 13, 60), (998, 60, 13, 60), (1894, 52, 13, 40), (77, 461, 21, 100),
          (151, 1203, 30, 60)]
+# CTAs of 5 and 7 columns over three and four column groups, whose first then has one column: the
+# second group's first column is the left edge's second one
+GRIDS += [(60, 560, 21, 60), (300, 900, 21, 60), (470, 620, 21, 60)]
 
 
 @pytest.mark.parametrize("history", [0, 1])
