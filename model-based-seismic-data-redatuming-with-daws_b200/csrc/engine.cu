@@ -1100,7 +1100,8 @@ int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> m
           nsta = std::max(nsta, n1);
         }
       if (nsta > 60000) return 0;
-      const int occ = resident_occupancy(mode, fp16, rho, C, RB, resident_smem(C, RB, pts, m, nsta, quads));
+      const int occ = resident_occupancy(mode, fp16, rho, false, C, RB,
+                                         resident_smem(C, RB, false, pts, m, nsta, quads));
       ok = ok && occ * h->sms >= (g.n2e + C - 1) / C;
     }
     if (ok) return C;
@@ -1145,6 +1146,7 @@ void* zeroed(daw_handle* h, const std::string& name, size_t bytes) {
 // Shape of a batch's runs of `mode` on chip: the tables and stages are sized for
 // the largest of its shots, active or not.
 struct ResidentShape {
+  bool ps = false;  // p in shared memory
   int G = 0, RB = 0, pts = 0, m = 0, nsta = 0, quads = 0, occ = 0;
   int room = 0;  // shots whose CTAs are resident together
 };
@@ -1167,9 +1169,17 @@ ResidentShape resident_shape(daw_handle* h, const Batch& b, int mode) {
     s.quads = std::max(s.quads, q);
   }
   if (!stage) s.quads = 0;
-  s.occ = resident_occupancy(mode == FM_STAGE_B_ES ? FM_STAGE_B : mode, h->opt.history_fp16 != 0,
-                             h->md.rbw1 != nullptr, b.res_cols, s.RB,
-                             resident_smem(b.res_cols, s.RB, s.pts, s.m, s.nsta, s.quads));
+  const int kmode = mode == FM_STAGE_B_ES ? FM_STAGE_B : mode;
+  auto occupancy = [&](bool ps) {
+    return resident_occupancy(kmode, h->opt.history_fp16 != 0, h->md.rbw1 != nullptr, ps, b.res_cols, s.RB,
+                              resident_smem(b.res_cols, s.RB, ps, s.pts, s.m, s.nsta, s.quads));
+  };
+  s.occ = occupancy(false);
+  // where it has room: stage B 151 x 461 3.04 to 2.68 us a step, 647 x 1533 6.84 to
+  // 6.59, 301 x 703 the same; both stages with FP32 histories 3.40 to 3.21 and 3.24
+  // to 2.80.  The forward run gains nothing and stage A with FP16 histories loses
+  // (registers spill: 3.7 to 4.2): they have no such variant.
+  s.ps = occupancy(true) >= s.occ;
   s.room = s.occ * h->sms / s.G;
   return s;
 }
@@ -1268,6 +1278,7 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
     return mode == FM_FWD ? c.srctab.dev : mode == FM_STAGE_A ? c.rectab.dev : ResidentInj{};
   };
   const ResidentShape shape = resident_shape(h, b, mode);
+  L.ps = shape.ps;
   L.inj_pts = shape.pts;
   L.inj_m = shape.m;
   L.inj_sta = shape.nsta;

@@ -47,6 +47,7 @@ struct ResidentShot {
 
 struct ResidentLaunch {
   int C, G, RB, groups;         // columns per CTA, CTAs per shot, 128-row blocks, shots
+  bool ps;                      // p in shared memory
   int CG, CW;                   // column groups and columns of a group (resident_launch)
   ulonglong2* halo;             // [phase][parity][cta][3][RB * 32][2]
   unsigned long long* slots;    // 72 words a CTA: stage A's maxima and their results
@@ -62,11 +63,11 @@ struct ResidentLaunch {
 };
 
 // Dynamic shared memory of a CTA.
-size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta, int quads);
+size_t resident_smem(int C, int RB, bool ps, int inj_pts, int inj_m, int inj_sta, int quads);
 // Warps of a CTA: column groups and columns per group.
-void resident_groups(int C, int RB, int* cg, int* cw);
+void resident_groups(int C, int RB, bool ps, int* cg, int* cw);
 // CTAs per SM of (mode, fp16, density) with that much shared memory; 0 when it does not fit.
-int resident_occupancy(int mode, bool fp16, bool rho, int C, int RB, size_t smem);
+int resident_occupancy(int mode, bool fp16, bool rho, bool ps, int C, int RB, size_t smem);
 cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaunch& L, int mode,
                             bool fp16, cudaStream_t st);
 // Fills the injection tables of a station map for the CTAs' headers.

@@ -49,8 +49,8 @@
 // neighbours' words waited for inside the edge column after what does not need
 // them (stage A 3.9 us against 3.7 at 151 x 461: registers spill).
 // Measured per shot step against the split kernels (B200, FP16 histories):
-// 751 x 2301 (17 columns a CTA) forward 7.1 us against 20.1, stage A 10.8
-// against 20.7-23.0, stage B 9.1 against 19.7-24.7; 151 x 461 (4 columns)
+// 751 x 2301 (17 columns a CTA) forward 7.0 us against 20.1, stage A 10.7
+// against 20.7-23.0, stage B 8.7 against 19.7-24.7; 151 x 461 (4 columns)
 // 2.4-3.7 us against 12-15.
 #include "resident.cuh"
 #include "tma.cuh"
@@ -384,9 +384,9 @@ __device__ __forceinline__ void sync_cta() {
 
 // Shared-memory layout (offsets in bytes, 16-byte aligned sections).
 struct Lay {
-  int fld, halo, edge, col, row, tcd, term, tsta, tkap, amp, stage, misc, total;
+  int fld, halo, edge, col, row, tcd, term, tsta, tkap, amp, stage, p, misc, total;
 };
-__host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, int quads) {
+__host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, int quads, bool ps) {
   Lay l;
   int o = 0;
   auto take = [&](int bytes) {
@@ -407,27 +407,39 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, i
   l.tkap = take(pts * 4);
   l.amp = take(2 * (nsta + 1) * 4);  // amplitudes of one step and the next
   l.stage = take(quads * C * 16);    // pressure of the gather rectangles [quad][column]
+  l.p = take(ps ? RB * (C + 3) * 512 : 0);  // [row block][column -1 .. C + 1][lane] quads of p
   l.misc = take(64 * 4 + 16);
   l.total = o;
   return l;
 }
-// Tensor-memory columns per row block of a quadrant: px, pz of the grid columns
-// -1 .. C + 1 (those outside 0 .. C - 1 hold the neighbours' p), kappa of 0 .. C - 1.
-__host__ __device__ inline int tm_words(int C, int RB) { return (RB + 3) / 4 * ((C + 3) * 8 + C * 4); }
-__host__ __device__ inline int tm_alloc(int C, int RB) {
+// Where p is, and with it which warps may share a row block.  Warp w reaches the
+// quadrant w % 4 of the tensor memory only, and at the borders of its columns it
+// reads p of the other column groups' warps.
+// - In tensor memory: a row block's warps share a quadrant, so the column groups
+//   are a multiple of 4 warps apart and the extra warp is in a gap or at the end.
+//   Five to seven row blocks load the four SM quadrants unevenly, one to three
+//   leave some idle.
+// - In shared memory too (PS, where it has room: 512 bytes per column and row
+//   block): tensor memory is private to a warp and the warps fill the quadrants
+//   in turn.  Stage B 151 x 461 3.04 to 2.68 us a step.
+__host__ __device__ inline int group_warps(int RB, bool ps) { return ps ? RB : (RB + 3) / 4 * 4; }
+__host__ __device__ inline int cta_warps(int RB, int CG, bool ps) {
+  return !ps && RB % 4 ? CG * group_warps(RB, ps) : CG * group_warps(RB, ps) + 1;
+}
+__host__ __device__ inline int aux_warp(int RB, int CG, bool ps) {
+  return !ps && RB % 4 ? RB : CG * group_warps(RB, ps);
+}
+// Tensor-memory columns.  p in tensor memory: per row block of a quadrant px, pz
+// of the grid columns -1 .. C + 1 (those outside 0 .. C - 1 hold the neighbours'
+// p), kappa of 0 .. C - 1; else per warp of a quadrant px, pz and kappa of its CW
+// columns.
+__host__ __device__ inline int tm_words(int C, int RB, int CG, int CW, bool ps) {
+  return ps ? (RB * CG + 3) / 4 * (CW * 12) : (RB + 3) / 4 * ((C + 3) * 8 + C * 4);
+}
+__host__ __device__ inline int tm_alloc(int C, int RB, int CG, int CW, bool ps) {
   int n = 32;
-  while (n < tm_words(C, RB)) n *= 2;
+  while (n < tm_words(C, RB, CG, CW, ps)) n *= 2;
   return n;
-}
-// Warps: CG column groups of RB row blocks, the groups a multiple of 4 warps
-// apart (a row block's warps share a quadrant), and the extra warp in a gap or
-// at the end.
-__host__ __device__ inline int group_warps(int RB) { return (RB + 3) / 4 * 4; }
-__host__ __device__ inline int cta_warps(int RB, int CG) {
-  return RB % 4 ? CG * group_warps(RB) : CG * group_warps(RB) + 1;
-}
-__host__ __device__ inline int aux_warp(int RB, int CG) {
-  return RB % 4 ? RB : CG * group_warps(RB);
 }
 
 // The injection terms ((c dt) amp) kappa of one step, by thread t of nt.
@@ -448,7 +460,7 @@ __device__ __forceinline__ void inj_terms(unsigned char* sm, const Lay& l, int p
   }
 }
 
-template <int MODE, bool FP16, bool RHO>
+template <int MODE, bool FP16, bool RHO, bool PS>
 __global__ void __launch_bounds__(32 * kResWarps, 1)
     k_resident(const __grid_constant__ Grid g, const __grid_constant__ ModelDev md,
                const __grid_constant__ ResidentLaunch L) {
@@ -459,14 +471,14 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   using HT = typename HQ::T;
   extern __shared__ __align__(16) unsigned char sm[];
   const int C = L.C, G = L.G, RB = L.RB;
-  const Lay l = layout(C, RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads);
+  const Lay l = layout(C, RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads, PS);
   const int grp = blockIdx.x / G, b = blockIdx.x - grp * G;
   const ResidentShot& S = L.shot[grp];
   // the warp index from a shuffle: the compiler then knows that it, and all
   // control that follows from it, is uniform over the warp
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(kAll, tid >> 5, 0);
-  const int rb = warp % group_warps(RB), cg = warp / group_warps(RB);  // row block, column group
-  const bool aux = warp == aux_warp(RB, L.CG);
+  const int rb = warp % group_warps(RB, PS), cg = warp / group_warps(RB, PS);  // row block, column group
+  const bool aux = warp == aux_warp(RB, L.CG, PS);
   const bool comp = !aux && rb < RB && cg < L.CG;  // else an idle warp: barriers only
   const int c0 = b * C, i1 = 128 * rb + 4 * lane;
   const int npml = g.npml, ld = g.ld;
@@ -483,6 +495,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   const u64* const FU = lane > 0 ? &(F + 31)->b : rb > 0 ? &(F + 63 - BS)->b : &(F + 32)->a;
   const float* const FD = reinterpret_cast<const float*>(
       lane < 31 ? F + 33 : rb < RB - 1 ? F + 1 + BS : F + 32) + (lane == 31 && rb >= RB - 1 ? 3 : 0);
+  Q4* const PP = reinterpret_cast<Q4*>(sm + l.p) + (comp ? rb : 0) * (C + 3) * 32 + 32 + lane;  // PS: p of column j at 32 j
   u64* const ED = reinterpret_cast<u64*>(sm + l.edge) + (rb + 1) * C * 2;
   ulonglong2* const CF = reinterpret_cast<ulonglong2*>(sm + l.col);
   ulonglong2* const SH = reinterpret_cast<ulonglong2*>(sm + l.halo) + (comp ? rb : 0) * 256 + 2 * lane;
@@ -500,7 +513,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   const int im = L.inj_m;
 
   // ---- set-up
-  const unsigned tcols = (unsigned)tm_alloc(C, RB);
+  const unsigned tcols = (unsigned)tm_alloc(C, RB, L.CG, L.CW, PS);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(TB)),
@@ -511,8 +524,11 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   sync_cta();
   // px, pz of column j: TP + 8 j (lane 32 (warp % 4) of the allocation)
   const unsigned TQ = __shfl_sync(kAll, *TB, 0) + ((unsigned)(warp & 3) << 21);
-  const unsigned TP = TQ + (rb >> 2) * (C + 3) * 8 + 8;
-  const unsigned TK = TQ + group_warps(RB) / 4 * (C + 3) * 8 + (rb >> 2) * C * 4;  // kappa: TK + 4 j
+  const unsigned TW = TQ + (warp >> 2) * L.CW * 12;  // PS: the warp's records
+  const unsigned TP = PS ? TW - 8 * clo : TQ + (rb >> 2) * (C + 3) * 8 + 8;
+  // kappa: TK + 4 j
+  const unsigned TK = PS ? TW + 8 * L.CW - 4 * clo
+                         : TQ + group_warps(RB, PS) / 4 * (C + 3) * 8 + (rb >> 2) * C * 4;
   {
     const int off = kF ? 2 : 3;
     const int hi1 = g.n1e - off, hi2 = g.n2e - off;
@@ -582,7 +598,12 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           sts4(F + FS * j + 32, kZero4);
         }
       __syncwarp();
-      if (cg == 0) {
+      if (PS && cg == 0) {
+        sts4(PP - 32, kZero4);
+        sts4(PP + 32 * C, kZero4);
+        sts4(PP + 32 * C + 32, kZero4);
+      }
+      if (!PS && cg == 0) {
         tm_st(TP - 8, kZero4, kZero4);
         tm_st(TP + 8 * C, kZero4, kZero4);
         tm_st(TP + 8 * C + 8, kZero4, kZero4);
@@ -626,7 +647,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   };
   if (aux) fetch_amp(first);
   // the warps but the extra one
-  const int it0 = tid - (warp > aux_warp(RB, L.CG) ? 32 : 0), itn = blockDim.x - 32;
+  const int it0 = tid - (warp > aux_warp(RB, L.CG, PS) ? 32 : 0), itn = blockDim.x - 32;
   if (ipts > 0 && !aux) inj_terms(sm, l, ipts, im, amp(first - 1), it0, itn);
 
   const u64 nz = L.nz;
@@ -830,6 +851,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         Q4* f = F + FS * j;
         const u64* fu = FU + 2 * FS * j;
         const float* fd = FD + 4 * FS * j;
+        Q4* pp = PP + 32 * j;
         const ulonglong2* cf = CF + 2 * j;
         u64* ed = ED + 2 * j;
         unsigned tp = TP + 8 * j, tk = TK + 4 * j, ho = (unsigned)((hoff + j * n1h) * kEs);
@@ -894,6 +916,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           }
           tm_st(tp + 8 * k, px, pz);
           const Q4 p = add4(px, pz);
+          if (PS) sts4(pp + 32 * k, p);
           sts_if(ed + 2 * k, p.a, top);
           sts_if(ed + 2 * k + 1, p.b, bottom);
           if (kA && (ph & (1u << k))) lmax = amax(lmax, p);
@@ -935,6 +958,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           sp0 += 4;
           sp1 += 4;
           fd += 16 * FS;
+          pp += 4 * 32;
           cf += 8;
           ed += 8;
           tp += 32;
@@ -999,6 +1023,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       ulonglong2* const hout = hmine + (size_t)(2 + (it & 1)) * hpar;  // phase 1: vx words
       const ulonglong2* const hin = hmine + (size_t)(it & 1) * hpar;   // p words
       auto pload = [&](int jj) {
+        if (PS) return lds4(PP + 32 * jj);
         Q4 x, z;
         tm_ld(TP + 8 * jj, x, z);
         return add4(x, z);
@@ -1021,21 +1046,31 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       auto put_right = [&]() {
         Q4 r[2];
         halo_get(SH + 128, hin + hcta + hcol, hcol, tag, poll, r);
-        tm_st(TP + 8 * C, r[0], kZero4);
-        tm_st(TP + 8 * C + 8, r[1], kZero4);
-        tm_wait_st();
+        if (PS) {
+          sts4(PP + 32 * C, r[0]);
+          sts4(PP + 32 * C + 32, r[1]);
+        } else {
+          tm_st(TP + 8 * C, r[0], kZero4);
+          tm_st(TP + 8 * C + 8, r[1], kZero4);
+          tm_wait_st();
+        }
       };
       auto put_left = [&]() {
         if (!lhalo) return;
         Q4 h[1];
         halo_get(SH, hin - hcta, hcol, tag, poll, h);
-        tm_st(TP - 8, h[0], kZero4);
-        tm_wait_st();
+        if (PS) {
+          sts4(PP - 32, h[0]);
+        } else {
+          tm_st(TP - 8, h[0], kZero4);
+          tm_wait_st();
+        }
       };
       // Columns [j, je), as in the pressure half step.
       auto columns = [&](int j, int je) {
         Q4* f = F + FS * j;
         const ulonglong2* cf = CF + 2 * j + 1;
+        const Q4* pp = PP + 32 * (j + 2);
         const u64* ed = ED + 2 * j;
         unsigned tp = TP + 8 * (j + 2), ho = (unsigned)((hoff + j * n1h) * kEs);
         unsigned ev = events >> j, ot = outs >> j, ph = phys >> j, src = lphys >> j;
@@ -1054,8 +1089,12 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           lds_if(n0, n1, reinterpret_cast<const float*>(ed + 2 * k + 2 * C), bottom);
           Q4 vx = lds4(f + FS * k), vz = lds4(f + FS * k + 32), qx, qz;
           const ulonglong2 c2 = cf[2 * k];
-          tm_ld(tp + 8 * k, qx, qz);
-          w3 = add4(qx, qz);
+          if (PS) {
+            w3 = lds4(pp + 32 * k);
+          } else {
+            tm_ld(tp + 8 * k, qx, qz);
+            w3 = add4(qx, qz);
+          }
           Q4 k2{c2.y, c2.y}, k1 = bw1, bu = kZero4;
           if (RHO) {
             const size_t o = (size_t)min(c0 + j + k, g.n2e - 1) * ld + min(i1, ld - 4);
@@ -1129,6 +1168,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           cf += 8;
           ed += 8;
           tp += 32;
+          pp += 4 * 32;
           ho += 4 * hstep;
           ev >>= 4;
           ot >>= 4;
@@ -1337,14 +1377,15 @@ __global__ void __launch_bounds__(32 * kGatherWarps)
 }
 
 template <typename F>
-void with_kernel(int mode, bool fp16, bool rho, F&& f) {
+void with_kernel(int mode, bool fp16, bool rho, bool ps, F&& f) {
   auto pick = [&](auto m, auto h) {
     constexpr int M = decltype(m)::value;
     constexpr bool H = decltype(h)::value;
-    if (rho)
-      f(k_resident<M, H, true>);
-    else
-      f(k_resident<M, H, false>);
+    constexpr bool P = M == FM_STAGE_B || (M == FM_STAGE_A && !H);  // the modes that have it
+    if (ps && P)
+      rho ? f(k_resident<M, H, true, P>) : f(k_resident<M, H, false, P>);
+    else if (!ps)
+      rho ? f(k_resident<M, H, true, false>) : f(k_resident<M, H, false, false>);
   };
   using std::false_type;
   using std::integral_constant;
@@ -1369,32 +1410,34 @@ constexpr int kTmCols = 512;
 
 }  // namespace
 
-size_t resident_smem(int C, int RB, int inj_pts, int inj_m, int inj_sta, int quads) {
-  const int tw = tm_words(C, RB);
-  if (tw > kTmCols) return kMaxSmem + 1;
-  // No more CTAs may be resident on an SM than its tensor memory holds: shared
-  // memory is padded until it admits just as many (an allocation that does not
-  // fit would block inside the kernel).
-  const size_t n = kTmCols / tm_alloc(C, RB);
-  const size_t floor_bytes = kMaxSmem / (n + 1) + 128;
-  return std::max((size_t)layout(C, RB, inj_pts, inj_m, inj_sta, quads).total, floor_bytes);
-}
-
-void resident_groups(int C, int RB, int* cg, int* cw) {
-  const int most = RB % 4 ? kResWarps / group_warps(RB) : (kResWarps - 1) / group_warps(RB);
+void resident_groups(int C, int RB, bool ps, int* cg, int* cw) {
+  const int w = group_warps(RB, ps);
+  const int most = !ps && RB % 4 ? kResWarps / w : (kResWarps - 1) / w;
   *cg = std::max(1, std::min(most, C));
   *cw = (C + *cg - 1) / *cg;
   *cg = (C + *cw - 1) / *cw;
 }
 
-int resident_occupancy(int mode, bool fp16, bool rho, int C, int RB, size_t smem) {
+size_t resident_smem(int C, int RB, bool ps, int inj_pts, int inj_m, int inj_sta, int quads) {
+  int cg, cw;
+  resident_groups(C, RB, ps, &cg, &cw);
+  if (tm_words(C, RB, cg, cw, ps) > kTmCols) return kMaxSmem + 1;
+  // No more CTAs may be resident on an SM than its tensor memory holds: shared
+  // memory is padded until it admits just as many (an allocation that does not
+  // fit would block inside the kernel).
+  const size_t n = kTmCols / tm_alloc(C, RB, cg, cw, ps);
+  const size_t floor_bytes = kMaxSmem / (n + 1) + 128;
+  return std::max((size_t)layout(C, RB, inj_pts, inj_m, inj_sta, quads, ps).total, floor_bytes);
+}
+
+int resident_occupancy(int mode, bool fp16, bool rho, bool ps, int C, int RB, size_t smem) {
   if (smem > kMaxSmem || RB > kResRowBlocks) return 0;
-  int n = 0, cg, cw;
-  resident_groups(C, RB, &cg, &cw);
-  with_kernel(mode, fp16, rho, [&](auto k) {
+  int n = 0, cg, cw;  // n stays 0 for a mode without the variant
+  resident_groups(C, RB, ps, &cg, &cw);
+  with_kernel(mode, fp16, rho, ps, [&](auto k) {
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 32 * cta_warps(RB, cg), smem) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 32 * cta_warps(RB, cg, ps), smem) !=
             cudaSuccess) {
       cudaGetLastError();
       n = 0;
@@ -1409,9 +1452,9 @@ cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaun
   cfg.gridDim = dim3(L.G * L.groups);
   ResidentLaunch P = L;
   P.nz = kNegZero2;
-  resident_groups(L.C, L.RB, &P.CG, &P.CW);
-  cfg.blockDim = dim3(32 * cta_warps(L.RB, P.CG));
-  cfg.dynamicSmemBytes = resident_smem(L.C, L.RB, L.inj_pts, L.inj_m, L.inj_sta, L.quads);
+  resident_groups(L.C, L.RB, L.ps, &P.CG, &P.CW);
+  cfg.blockDim = dim3(32 * cta_warps(L.RB, P.CG, L.ps));
+  cfg.dynamicSmemBytes = resident_smem(L.C, L.RB, L.ps, L.inj_pts, L.inj_m, L.inj_sta, L.quads);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeCooperative;  // CTAs wait on one another: all are resident
@@ -1419,7 +1462,7 @@ cudaError_t resident_launch(const Grid& g, const ModelDev& m, const ResidentLaun
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaError_t e = cudaSuccess;
-  with_kernel(mode, fp16, m.rbw1 != nullptr,
+  with_kernel(mode, fp16, m.rbw1 != nullptr, L.ps,
               [&](auto k) { e = cudaLaunchKernelEx(&cfg, k, g, m, P); });
   return e;
 }
