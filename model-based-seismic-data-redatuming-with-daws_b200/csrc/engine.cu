@@ -265,6 +265,9 @@ struct daw_handle {
   int slot_datum = 0, slot_win = 0;
   bool slot_fp16 = false;
   unsigned res_tag = 1;  // next step tag of the on-chip time loops
+  // CTAs per SM of their kernels by (mode, FP16, density, p in shared memory, columns
+  // per CTA, row blocks, shared memory)
+  std::map<std::array<size_t, 7>, int> res_occ;
 };
 
 namespace {
@@ -1062,35 +1065,83 @@ int staged_quads(int C, const Box box[2]) {
   return q * C * 16 <= kStageBytes ? q : 0;
 }
 
+int res_occupancy(daw_handle* h, int mode, bool ps, int C, int RB, size_t smem) {
+  const bool fp16 = h->opt.history_fp16 != 0, rho = h->md.rbw1 != nullptr;
+  const std::array<size_t, 7> key{(size_t)mode, fp16, rho, ps, (size_t)C, (size_t)RB, smem};
+  const auto it = h->res_occ.find(key);
+  if (it != h->res_occ.end()) return it->second;
+  return h->res_occ[key] = resident_occupancy(mode, fp16, rho, ps, C, RB, smem);
+}
+
+// Estimates in us, the mean of forward, stage A and stage B steps (B200, grids of
+// 60 x 90 to 751 x 2301 points, 1 to 64 shots; to 15 % of the measured ones).
+// One step of an on-chip launch, whatever the number of its shots, from the columns a
+// warp walks; the launch of a shot's gathers after its loop takes kGatherUs.  One step
+// of n shots in the split kernels, which take them all in one launch: a latency and
+// the points' traffic, which overlap for few shots.
+double resident_step_us(int C, int RB) {
+  int cg, cw;
+  resident_groups(C, RB, false, &cg, &cw);
+  return std::max(2.9, 1.3 + 0.88 * cw);
+}
+constexpr double kGatherUs = 45.0;
+double split_step_us(const Grid& g, int n) {
+  const double points = n * (0.14 + 11.1e-6 * (double)g.n1e * g.n2e);
+  return std::max({12.0, 10.0 + 0.75 * points, 4.0 + points});
+}
+
 // Columns per CTA with which the batch's runs of `modes` can stay on chip, or
-// 0.  The rule is on the grid (its points fit the SMs' registers and shared
+// 0.  The rule is on the grid (its points fit the SMs' shared and tensor
 // memory), on where the stations inject (clear of the rows and columns that
 // are never updated), on how many entries their tables have (they fit beside
 // the fields) and on how much of the grid the gathers read.
+//
+// A launch holds as many shots as have room; a batch takes several launches one
+// after the other.  Fewer columns per CTA shorten a step, more let a launch hold
+// more shots, so a batch gets the width with the least (launches x step), and
+// the split kernels where they are estimated faster: a grid that is small beside the
+// chip, many times over.  us per shot step, forward / stage A / stage B, with the
+// narrowest CTAs, the width chosen, and the split kernels (FP16 histories):
+//   151 x 461, 16 shots  2.7 / 4.0 / 3.0  1.1 / 1.5 / 1.1  1.7 / 1.7 / 1.7
+//   301 x 151, 32 shots  1.6 / 1.8 / 1.8  0.6 / 0.6 / 0.5  1.0 / 1.0 / 1.0
+//   301 x 703, 8 shots   3.1 / 4.2 / 3.8  1.6 / 2.1 / 1.6  3.8 / 3.5 / 3.3
+//   77 x 201, 16 shots   1.3 / 1.8 / 1.5  0.6 / 0.6 / 0.3  1.1 / 0.9 / 0.9
+//   60 x 90, 64 shots    0.7 / 0.9 / 0.9  0.4 / 0.4 / 0.3  0.4 / 0.4 / 0.4
 int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> modes) {
   const Grid& g = h->g;
   const int RB = (g.n1e + 127) / 128;
   if (!resident_family(h) || RB > kResRowBlocks || g.npml < 3 || g.n2e < 8) return 0;
   if (g.ofs == 1 && g.npml % 128 == 0) return 0;  // vz(npml) and vz(npml+1) in different warps
-  const bool fp16 = h->opt.history_fp16 != 0, rho = h->md.rbw1 != nullptr;
-  for (const ShotCtx* c : b.shots)
-    for (int mode : modes) {
+  int n = 0;  // shots to run
+  std::vector<std::array<Box, 2>> boxes;  // of each mode's shots
+  for (const ShotCtx* c : b.shots) n += c->active ? 1 : 0;
+  for (int mode : modes)
+    for (const ShotCtx* c : b.shots) {
       if (mode == FM_FWD && c->type_src != 0) return 0;
-      Box box[2];
+      boxes.emplace_back();
+      Box* box = boxes.back().data();
       gather_boxes(h, b, *c, mode, box);
       if ((box[0].elems() + box[1].elems()) * sizeof(float) > kRectStepBytes) return 0;
     }
+  int best = 0;
+  double gathers = 0;  // of a shot and mode
+  for (const auto& x : boxes)
+    for (const Box& k : x) gathers += k.elems() ? 1.0 / boxes.size() : 0.0;
+  double best_us = HUGE_VAL;
+  if (n > 1) best_us = split_step_us(g, n) - n * gathers * kGatherUs / b.max_nt;
   for (int C = std::max(4, (g.n2e + h->sms - 1) / h->sms); C <= kResCols; ++C) {
-    bool ok = true;
-    for (int mode : modes) {
-      int pts = 0, m = 0, nsta = 0, quads = 0;
-      for (const ShotCtx* c : b.shots) {
-        Box box[2];
-        gather_boxes(h, b, *c, mode, box);
-        quads = std::max(quads, staged_quads(C, box));
-      }
-      if (mode == FM_FWD || mode == FM_STAGE_A)
+    const int G = (g.n2e + C - 1) / C;
+    const double step_us = resident_step_us(C, RB);
+    auto us = [&](int room) { return (std::max(n, 1) + room - 1) / room * step_us; };
+    int room = kResShots;
+    for (int pass = 0; pass < 2 && room > 0; ++pass) {  // without the stations' share of the memory, then with it
+      size_t k = 0;
+      for (int mode : modes) {
+        int pts = 0, m = 0, nsta = 0, quads = 0;
         for (const ShotCtx* c : b.shots) {
+          if (pass == 0) break;
+          quads = std::max(quads, staged_quads(C, boxes[k++].data()));
+          if (mode != FM_FWD && mode != FM_STAGE_A) continue;
           int p1, m1, n1;
           if (!resident_heads(g, mode == FM_FWD ? c->srcinfo : c->recinfo, C,
                               mode == FM_FWD ? 2 : 3, nullptr, &p1, &m1, &n1))
@@ -1099,14 +1150,18 @@ int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> m
           m = std::max(m, m1);
           nsta = std::max(nsta, n1);
         }
-      if (nsta > 60000) return 0;
-      const int occ = resident_occupancy(mode, fp16, rho, false, C, RB,
-                                         resident_smem(C, RB, false, pts, m, nsta, quads));
-      ok = ok && occ * h->sms >= (g.n2e + C - 1) / C;
+        if (nsta > 60000) return 0;
+        room = std::min(room, res_occupancy(h, mode, false, C, RB,
+                                            resident_smem(C, RB, false, pts, m, nsta, quads)) * h->sms / G);
+      }
+      if (room > 0 && us(room) >= best_us) room = 0;  // no gain over a width (or the split kernels) before
     }
-    if (ok) return C;
+    if (room < 1) continue;
+    best = C;
+    best_us = us(room);
+    if (room >= n) break;  // more columns only make a step longer
   }
-  return 0;
+  return best;
 }
 
 // Injection tables of a shot's map for C columns per CTA (built once per shot
@@ -1171,8 +1226,8 @@ ResidentShape resident_shape(daw_handle* h, const Batch& b, int mode) {
   if (!stage) s.quads = 0;
   const int kmode = mode == FM_STAGE_B_ES ? FM_STAGE_B : mode;
   auto occupancy = [&](bool ps) {
-    return resident_occupancy(kmode, h->opt.history_fp16 != 0, h->md.rbw1 != nullptr, ps, b.res_cols, s.RB,
-                              resident_smem(b.res_cols, s.RB, ps, s.pts, s.m, s.nsta, s.quads));
+    return res_occupancy(h, kmode, ps, b.res_cols, s.RB,
+                         resident_smem(b.res_cols, s.RB, ps, s.pts, s.m, s.nsta, s.quads));
   };
   s.occ = occupancy(false);
   // where it has room: stage B 151 x 461 3.04 to 2.68 us a step, 647 x 1533 6.84 to
