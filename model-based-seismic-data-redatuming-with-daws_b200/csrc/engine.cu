@@ -50,10 +50,18 @@ void check_launch(const char* what) {
   if (e != cudaSuccess) throw DawError{DAW_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)};
 }
 
-// Grow-only named device buffers owned by a handle.
+// Grow-only named device buffers owned by a handle.  What the on-chip time loops
+// keep between runs ("resident.") is given back where another buffer needs its
+// memory; they make it anew when the next run is planned.
 struct Pool {
   std::map<std::string, DevBuf> bufs;
   size_t total = 0;
+  Pool* lender = this;       // the pool that has those
+  unsigned given_back = 0;   // times that they went
+  void give_back() {
+    release_prefix("resident.");
+    ++given_back;
+  }
   void* get(const std::string& name, size_t bytes) {
     if (bytes == 0) bytes = 16;
     DevBuf& b = bufs[name];
@@ -64,7 +72,13 @@ struct Pool {
       }
       b.p = nullptr;
       b.bytes = 0;
-      if (cudaMalloc(&b.p, bytes) != cudaSuccess) {
+      cudaError_t e = cudaMalloc(&b.p, bytes);
+      if (e != cudaSuccess && name.compare(0, 9, "resident.") != 0) {
+        cudaGetLastError();
+        lender->give_back();
+        e = cudaMalloc(&b.p, bytes);
+      }
+      if (e != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
         throw DawError{DAW_ERR_OOM, "device allocation of " + std::to_string(bytes) +
@@ -95,6 +109,7 @@ struct Pool {
       if (kv.second.p) cudaFree(kv.second.p);
     bufs.clear();
     total = 0;
+    ++given_back;
   }
 };
 
@@ -147,6 +162,7 @@ struct MapInfo {
 // A station map's injection tables for CTAs of C columns (resident.cuh).
 struct ResTables {
   int C = 0;
+  unsigned given_back = 0;  // Pool::given_back when they were made
   ResidentInj dev{};
 };
 
@@ -1168,13 +1184,13 @@ int resident_columns(daw_handle* h, const Batch& b, std::initializer_list<int> m
 // and width).
 void make_tables(daw_handle* h, const ShotCtx& c, const MapInfo& info, const InjMapDev& map, int C,
                  const char* name, ResTables* t) {
-  if (t->C == C) return;
+  if (t->C == C && t->given_back == h->pool.given_back) return;
   std::vector<int4> heads;
   ResidentInj d{};
   resident_heads(h->g, info, C, 2, &heads, &d.pts, &d.m, &d.nsta);
   const int G = (int)heads.size();
   if (d.pts > 0) {
-    const std::string p = c.tag + name;
+    const std::string p = "resident." + c.tag + name;
     int4* head = h->pool.get_t<int4>(p + ".head", G);
     const size_t n = (size_t)G * d.pts;
     float* cd = h->pool.get_t<float>(p + ".cd", n * d.m);
@@ -1187,6 +1203,7 @@ void make_tables(daw_handle* h, const ShotCtx& c, const MapInfo& info, const Inj
     d.head = head; d.cd = cd; d.sta = sta; d.kap = kap;
   }
   t->C = C;
+  t->given_back = h->pool.given_back;
   t->dev = d;
 }
 
@@ -1240,8 +1257,9 @@ ResidentShape resident_shape(daw_handle* h, const Batch& b, int mode) {
 }
 
 // Buffers of a batch's runs of `mode` on chip, for as many shots as run
-// together: halo words, maxima, and the rectangle buffer, which takes less (the
-// loops then run in shorter launches) where memory is short of its usual size.
+// together: halo words, maxima, and the rectangle buffer, which takes at most half
+// of the memory that is free (the loops then run in shorter launches), since what is
+// allocated later and not by the pool, graphs and kernels' code, needs some too.
 // Throws DAW_ERR_OOM when one step of the rectangles does not fit either.
 void reserve_resident(daw_handle* h, const Batch& b, int mode) {
   const ResidentShape s = resident_shape(h, b, mode);
@@ -1258,14 +1276,15 @@ void reserve_resident(daw_handle* h, const Batch& b, int mode) {
   size_t one = 0;  // the largest group's step
   for (size_t i = 0; i < q; ++i) one += elems[i] * sizeof(float);
   if (!one) return;
-  for (size_t bytes = std::max(one, std::min(kRectBytes, one * b.max_nt));; bytes = std::max(one, bytes / 2)) {
-    try {
-      h->pool.get("resident.rect", bytes);
-      return;
-    } catch (const DawError& e) {
-      if (e.code != DAW_ERR_OOM || bytes == one) throw;
-    }
-  }
+  const size_t bytes = std::max(one, std::min(kRectBytes, one * b.max_nt));
+  const size_t held = h->pool.bufs["resident.rect"].bytes;
+  if (held >= bytes) return;
+  size_t free_b = 0, total_b = 0;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  const size_t room = (free_b + held) / 2;
+  if (held >= std::max(one, room)) return;
+  if (one > room) throw DawError{DAW_ERR_OOM, "no device memory for the on-chip loops' rectangles"};
+  h->pool.get("resident.rect", std::min(bytes, room));
 }
 
 // From global memory, one kernel per step moves 36 bytes a point and step and two
@@ -1291,18 +1310,21 @@ bool plan_resident(daw_handle* h, Batch& b, std::initializer_list<int> modes) {
   b.step = large_grid(h);
   b.res_cols = resident_columns(h, b, modes);
   if (!b.res_cols) return false;
+  bool fits = true;
   try {
     for (ShotCtx* c : b.shots)
       for (int mode : modes) {
         if (mode == FM_FWD) make_tables(h, *c, c->srcinfo, c->srcmap, b.res_cols, "srctab", &c->srctab);
         if (mode == FM_STAGE_A) make_tables(h, *c, c->recinfo, c->recmap, b.res_cols, "rectab", &c->rectab);
       }
-    for (int mode : modes) {
-      if (resident_shape(h, b, mode).room < 1) return false;
-      reserve_resident(h, b, mode);
-    }
+    for (int mode : modes)
+      if ((fits = fits && resident_shape(h, b, mode).room >= 1)) reserve_resident(h, b, mode);
   } catch (const DawError& e) {
     if (e.code != DAW_ERR_OOM) throw;
+    fits = false;
+  }
+  if (!fits) {
+    h->pool.give_back();
     return false;
   }
   b.resident = true;
@@ -1595,7 +1617,14 @@ void run_fused(daw_handle* h, Batch& b, int mode, const Window* w = nullptr) {
         body();
         CK(cudaStreamEndCapture(h->st, &graph));
         cudaGraphExec_t exec;
-        CK(cudaGraphInstantiate(&exec, graph, 0));
+        cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+        if (e == cudaErrorMemoryAllocation) {
+          cudaGetLastError();
+          h->pool.give_back();
+          e = cudaGraphInstantiate(&exec, graph, 0);
+        }
+        if (e != cudaSuccess) cudaGraphDestroy(graph);
+        CK(e);
         cudaGraphDestroy(graph);
         it = h->graphs.emplace(key, exec).first;
       }
@@ -2363,7 +2392,8 @@ int admit_batch(daw_handle* h, int n, const daw_shot_desc* d, bool want_wf, int*
 void release_slots(daw_handle* h) {
   drop_graphs(h);
   h->slot_shapes.clear();
-  for (const char* p : {"slot", "shot", "mr", "batch."}) h->pool.release_prefix(p);
+  for (const char* p : {"slot", "shot", "mr", "batch.", "resident.shot"}) h->pool.release_prefix(p);
+  ++h->pool.given_back;  // the tables among them
 }
 
 // Per-slot buffers for a batch: those of the last batch where every shot fits the
@@ -2529,6 +2559,7 @@ int daw_create(daw_handle** out, int32_t device) {
     return DAW_ERR_CUDA;
   }
   apply_preset(h->opt, 1);
+  h->model_pool.lender = &h->pool;
   if (cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess) {
     cudaGetLastError();
     cudaStreamDestroy(h->st);
