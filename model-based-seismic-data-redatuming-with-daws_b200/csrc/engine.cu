@@ -2327,10 +2327,7 @@ void fetch_outputs(daw_handle* h, ShotCtx& c, daw_shot_out* o) {
 size_t admission_bytes(daw_handle* h) {
   size_t free_b = 0, total_b = 0;
   CK(cudaMemGetInfo(&free_b, &total_b));
-  size_t held = h->pool.total;  // less what the on-chip time loops keep between calls
-  for (const auto& kv : h->pool.bufs)
-    if (kv.first.compare(0, 9, "resident.") == 0) held -= kv.second.bytes;
-  return (size_t)((double)(free_b + held) * 0.92);
+  return (size_t)((double)(free_b + h->pool.total) * 0.92);
 }
 
 // Stage-A history window of a shot of nt steps (fused kernels only): 0 keeps

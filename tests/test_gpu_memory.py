@@ -45,3 +45,33 @@ def test_pipeline_with_little_memory(pkg):
             finally:
                 del held
                 torch.cuda.empty_cache()
+
+
+def admitted(pkg, h, nt, shot):
+    """History window of a record too long for the device."""
+    rec = np.asfortranarray(shot["rec"], np.int32)
+    s, dobs = np.zeros(nt, np.float32), np.zeros((nt, 1), np.float32)
+    d = (pkg.ShotDesc * 1)()
+    d[0].nt, d[0].nrec = nt, 1
+    d[0].s, d[0].dobs = (a.ctypes.data_as(C.POINTER(C.c_float)) for a in (s, dobs))
+    for k in range(5):
+        d[0].src_tab[k] = int(shot["src"][k])
+    one = np.asfortranarray(rec[:1])
+    d[0].rec_tab = one.ctypes.data_as(C.POINTER(C.c_int32))
+    n, win = C.c_int32(), C.c_int32()
+    assert pkg.lib().daw_admit_shots(h._h, 1, d, C.byref(n), C.byref(win)) == 0
+    assert n.value == 1 and 0 < win.value < nt
+    return win.value
+
+
+def test_admission_after_a_run(pkg):
+    """A run on chip keeps 512 MB of rectangles (177 steps of this grid's history); as
+    long a record is admitted after it as before, the device's own allocations
+    (a few MB, a step each 2.8 MB) aside."""
+    w, shot = workload(pkg, nrec=9)
+    with handle(pkg, w) as h:
+        h.submodeling_adjoint_esource_data(shot["dobs"][:40], shot["rec"])  # kernels loaded
+        before = admitted(pkg, h, 300000, shot)
+        h.submodeling(shot["s"], shot["src"], shot["rec"])
+        assert h.timing()["kernel_family"][0] == 2
+        assert admitted(pkg, h, 300000, shot) >= before - 20
