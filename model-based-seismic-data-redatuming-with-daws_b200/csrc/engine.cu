@@ -1455,16 +1455,16 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
       for (int i = 0; i < n; ++i) {
         ShotCtx& c = *act[g0 + i];
         const ResidentShot& S = L.shot[i];
-        const int ns = S.last - S.first + 1;
+        const int ns = S.last - S.first + 1, off = mode == FM_FWD ? 2 : 3;
         if (S.rect[0].buf) {
           float* out = mode == FM_FWD ? c.d_datar : c.op_out;
           const int rev = mode == FM_FWD ? 0 : c.op_reverse;
-          resident_gather(S.rect[0], c.rec, 0, g.n1e, 0, g.n2e, ns, out, c.nt,
+          resident_gather(g, S.rect[0], c.rec, off, 0, g.n1e, 0, g.n2e, ns, out, c.nt,
                           rev ? c.nt - S.first : S.first - 1, rev, h->st);
           h->tim.kernel_launches += 1;
         }
         if (S.rect[1].buf) {
-          resident_gather(S.rect[1], h->datum, g.npml, g.npml + g.n1, g.npml, g.npml + g.n2, ns,
+          resident_gather(g, S.rect[1], h->datum, off, g.npml, g.npml + g.n1, g.npml, g.npml + g.n2, ns,
                           mode == FM_FWD ? c.d_redF : c.d_redE, c.nt, S.first - 1, 0, h->st);
           h->tim.kernel_launches += 1;
         }

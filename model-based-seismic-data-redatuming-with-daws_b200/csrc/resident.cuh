@@ -75,10 +75,12 @@ void resident_tables(const Grid& g, const ModelDev& m, const InjMapDev& map, int
                      const int4* head, int pts, int mm, float* cd, unsigned short* sta, float* kap,
                      cudaStream_t st);
 // Hicks sums of a station set for steps 0 .. nsteps-1 of a rectangle buffer,
-// the support clipped to rows [lo1, hi1) and columns [lo2, hi2):
+// the support clipped to rows [lo1, hi1) and columns [lo2, hi2), and to the points that
+// are updated (`off` rows and columns at the far edges are not), which the others'
+// zeros add nothing to:
 // out[row(step) + nt * station], row = row0 + step, or row0 - step when reverse.
-void resident_gather(const ResidentRect& r, const StationsDev& st, int lo1, int hi1, int lo2,
-                     int hi2, int nsteps, float* out, int nt, int row0, int reverse,
+void resident_gather(const Grid& g, const ResidentRect& r, const StationsDev& st, int off, int lo1,
+                     int hi1, int lo2, int hi2, int nsteps, float* out, int nt, int row0, int reverse,
                      cudaStream_t s);
 
 }  // namespace daw

@@ -31,7 +31,10 @@
 // Rows 0, 1 and the last rows and columns are never updated and the caller
 // keeps sources away from them, so they stay zero: their update coefficients
 // are set to zero instead of branching.  The same holds for px and pz above the
-// free surface, where the pressure is zeroed.
+// free surface, where the pressure is zeroed.  (Once a value is not finite, zero times
+// it is not zero, and these points hold NaN.  The wavefield output has zeros there all
+// the same and the gathers leave them out; points that are updated get the same values
+// as with zeros there.)
 //
 // Arithmetic: the reference's separately rounded FP32 operations, two rows at
 // a time in packed (f32x2) instructions; bit-identical to the other kernels.
@@ -52,6 +55,8 @@
 // 751 x 2301 (17 columns a CTA) forward 7.0 us against 20.1, stage A 10.7
 // against 20.7-23.0, stage B 8.7 against 19.7-24.7; 151 x 461 (4 columns)
 // 2.4-3.7 us against 12-15.
+#include <algorithm>
+
 #include "resident.cuh"
 #include "tma.cuh"
 
@@ -932,10 +937,13 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
             if (S.wf && (ph & (1u << k))) {
               float* w = S.wf + (size_t)(it - 1) * g.int_elems() + (size_t)g.n1 * (c0 + j + k - npml) + (i1 - npml);
               const bool acc = S.wf_acc != 0;
-              if (rows & 1u) w[0] = acc ? fadd(w[0], v.x) : v.x;
-              if (rows & 2u) w[1] = acc ? fadd(w[1], v.y) : v.y;
-              if (rows & 4u) w[2] = acc ? fadd(w[2], v.z) : v.z;
-              if (rows & 8u) w[3] = acc ? fadd(w[3], v.w) : v.w;
+              const int top_zero = g.ofs == 1 ? npml - i1 : -1;  // the lane's last row of zeros
+              const float4 u = make_float4(top_zero < 0 ? v.x : 0.f, top_zero < 1 ? v.y : 0.f,
+                                           top_zero < 2 ? v.z : 0.f, top_zero < 3 ? v.w : 0.f);
+              if (rows & 1u) w[0] = acc ? fadd(w[0], u.x) : u.x;
+              if (rows & 2u) w[1] = acc ? fadd(w[1], u.y) : u.y;
+              if (rows & 4u) w[2] = acc ? fadd(w[2], u.z) : u.z;
+              if (rows & 8u) w[3] = acc ? fadd(w[3], u.w) : u.w;
               __syncwarp();
             }
           }
@@ -1337,8 +1345,8 @@ __global__ void __launch_bounds__(32 * kGatherWarps)
   const bool on = s < st.n;
   // 0-based first tap of the station; support clipped to [ra, rb) x [ca, cb)
   const int a0 = on ? st.ix1[s] - 1 - kRad : 0, b0 = on ? st.ix2[s] - 1 - kRad : 0;
-  const bool full = on && a0 >= ra && a0 + kTap <= rb && b0 >= ca && b0 + kTap <= cb;
-  const bool allfull = __all_sync(kAll, full || !on);
+  const int alo = max(0, ra - a0), ahi = min(kTap, rb - a0);
+  const bool allfull = __all_sync(kAll, (b0 >= ca && b0 + kTap <= cb) || !on);  // all columns
   for (int t0 = (blockIdx.y * kGatherWarps + warp) * kGatherSteps; t0 < nsteps;
        t0 += gridDim.y * kGatherWarps * kGatherSteps) {
     float acc[kGatherSteps] = {};
@@ -1348,7 +1356,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps)
       base[k] = r.buf + (size_t)min(t0 + k, nsteps - 1) * r.step;
     if (on) {
       if (allfull) {
-        for (int a = 0; a < kTap; ++a) {
+        for (int a = alo; a < ahi; ++a) {
           const size_t o = (size_t)(a0 + a - r.r0) * r.ld + (b0 - r.c0);
 #pragma unroll
           for (int q = 0; q < kTap; ++q) {
@@ -1358,7 +1366,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps)
           }
         }
       } else {
-        for (int a = max(0, ra - a0); a < kTap && a0 + a < rb; ++a)
+        for (int a = alo; a < ahi; ++a)
           for (int q = max(0, ca - b0); q < kTap && b0 + q < cb; ++q) {
             const float c = tl[(a + kTap * q) * 33 + lane];
             const size_t o = (size_t)(a0 + a - r.r0) * r.ld + (b0 + q - r.c0);
@@ -1473,10 +1481,14 @@ void resident_tables(const Grid& g, const ModelDev& m, const InjMapDev& map, int
   k_resident_tables<<<G, 256, 0, st>>>(g, m.kap, map, C, head, pts, mm, cd, sta, kap);
 }
 
-void resident_gather(const ResidentRect& r, const StationsDev& st, int lo1, int hi1, int lo2,
-                     int hi2, int nsteps, float* out, int nt, int row0, int reverse,
+void resident_gather(const Grid& g, const ResidentRect& r, const StationsDev& st, int off, int lo1,
+                     int hi1, int lo2, int hi2, int nsteps, float* out, int nt, int row0, int reverse,
                      cudaStream_t s) {
   if (st.n <= 0 || nsteps <= 0) return;
+  lo1 = std::max({lo1, 2, g.ofs == 1 ? g.npml + 1 : 0});
+  lo2 = std::max(lo2, 2);
+  hi1 = std::min(hi1, g.n1e - off);
+  hi2 = std::min(hi2, g.n2e - off);
   constexpr size_t smem = kTile * 33 * sizeof(float);
   cudaFuncSetAttribute(k_resident_gather, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int per = kGatherWarps * kGatherSteps;
