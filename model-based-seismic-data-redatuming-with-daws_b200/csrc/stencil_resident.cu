@@ -11,11 +11,12 @@
 //
 // Halo columns go from lane to lane of neighbouring CTAs through L2: the
 // writer stores (value, step tag) as one 64-bit word, so the reader's poll of
-// the data is also the wait and no fence or flag follows it.  A lane needs its
+// the data is also the wait and no fence or flag follows it.  Writer and reader use
+// relaxed accesses of gpu scope, whose 64-bit words are whole, and nothing else reads
+// the words.  A lane needs its
 // neighbour CTA's values of its own rows only, and only for the first two and
 // the last column; those columns are computed last in a half step, so the
-// words travel while the columns between are computed, and they are fetched
-// into shared memory a few columns ahead of their use.  Buffers alternate by
+// words travel while the columns between are computed.  Buffers alternate by
 // step parity: a CTA writes parity s only after it has read its neighbours'
 // words of step s - 1, which they store after their last read of step s - 2.
 // Rows couple neighbouring warps (vz through shared memory, p through warp
@@ -157,24 +158,25 @@ struct Poll {
   }
 };
 
-// N halo columns at p, p + stride, ...: `fetch` copies the lane's words to its
-// place in shared memory, early and without waiting; `get` checks their tags
-// there and polls the words themselves until all carry the tag.
-template <int N>
-__device__ __forceinline__ void halo_fetch(ulonglong2* sh, const ulonglong2* p, size_t stride) {
-#pragma unroll
-  for (int k = 0; k < 2 * N; ++k)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(sh + (k / 2) * 64 + (k & 1))),
-                 "l"(p + (k / 2) * stride + (k & 1))
-                 : "memory");
-}
-template <int N>
-__device__ __forceinline__ void halo_get(const ulonglong2* sh, const ulonglong2* p, size_t stride,
-                                         unsigned tag, Poll& w, Q4 (&v)[N]) {
-  asm volatile("cp.async.wait_all;" ::: "memory");
+// N halo columns at p, p + stride, ...: polled until all words carry the tag, between
+// the parts of a warp's columns (in the column code itself the wait is there four times
+// over: instruction cache).  us per step of forward / stage A / stage B, 751 x 2301 6.93
+// / 10.9 / 8.37, 301 x 703 2.59 / 4.12 / 3.42, 151 x 461 2.20 / 3.7 / 2.57.  Tried:
+// - in the column code 7.20 / 10.9 / 9.19, 2.57 / 4.2 / 3.86, 2.12 / 3.8 / 2.78;
+// - there, copied to shared memory a few columns ahead by cp.async, which is a weak access
+//   and races with the neighbour's store in the memory model: 7.13 / 10.7 / 8.78, 2.56 /
+//   4.2 / 3.49, 2.27 / 3.7 / 2.69;
+// - loaded a few columns ahead and put into shared memory by the lane, at once: 7.80 /
+//   11.6 / 9.62, 2.85 / 4.3 / 4.08, 2.40 / 3.9 / 3.18; at the end of the column: stage B
+//   11.5, 4.44, 3.51 (registers spill);
+// - copied by the extra warp: forward and stage B 10.6 / 12.1, 4.75 / 6.6, 3.56 / 5.0.
+template <int N, typename F>
+__device__ __forceinline__ void halo_get(const ulonglong2* p, size_t stride, unsigned tag, Poll& w,
+                                         Q4 (&v)[N], F&& meanwhile) {
   ulonglong2 x[2 * N];
 #pragma unroll
-  for (int k = 0; k < 2 * N; ++k) x[k] = sh[(k / 2) * 64 + (k & 1)];
+  for (int k = 0; k < 2 * N; ++k) x[k] = ll_load(p + (k / 2) * stride + (k & 1));
+  meanwhile();  // other loads
   for (int n = 0;; ++n) {
     bool ok = true;
 #pragma unroll
@@ -389,7 +391,7 @@ __device__ __forceinline__ void sync_cta() {
 
 // Shared-memory layout (offsets in bytes, 16-byte aligned sections).
 struct Lay {
-  int fld, halo, edge, col, row, tcd, term, tsta, tkap, amp, stage, p, misc, total;
+  int fld, edge, col, row, tcd, term, tsta, tkap, amp, stage, p, misc, total;
 };
 __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, int quads, bool ps) {
   Lay l;
@@ -402,7 +404,6 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, i
   // [row block][column -2 .. C][vx, vz][lane] quads; columns -2, -1 and C hold
   // the neighbours' vx
   l.fld = take(RB * (C + 3) * 1024);
-  l.halo = take(RB * 4096);          // [row block][2 left, 2 right columns][lane][2] halo words
   l.edge = take((RB + 2) * C * 16);  // [row block + 1][column][first, last pair of p]
   l.col = take(C * 32);              // [column][d2a, d2a, d2a1, d2a1, d2b, d2b, bw2, bw2]
   l.row = take(4 * RB * 512);        // d1a, d1a1, d1b, bw1
@@ -503,7 +504,6 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   Q4* const PP = reinterpret_cast<Q4*>(sm + l.p) + (comp ? rb : 0) * (C + 3) * 32 + 32 + lane;  // PS: p of column j at 32 j
   u64* const ED = reinterpret_cast<u64*>(sm + l.edge) + (rb + 1) * C * 2;
   ulonglong2* const CF = reinterpret_cast<ulonglong2*>(sm + l.col);
-  ulonglong2* const SH = reinterpret_cast<ulonglong2*>(sm + l.halo) + (comp ? rb : 0) * 256 + 2 * lane;
   Q4* const ROW = reinterpret_cast<Q4*>(sm + l.row) + rb * 32 + lane;
   const int NP = RB * 32;
   float* const TERM = reinterpret_cast<float*>(sm + l.term);
@@ -823,31 +823,27 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
       ulonglong2* const hout = hmine + (size_t)(it & 1) * hpar;  // phase 0: p words
       const ulonglong2* const hin = hmine + (size_t)(2 + ((it - 1) & 1)) * hpar;  // vx words
       // The warp's columns in order, those of the left edge (0 and 1) last: the
-      // neighbours' words are fetched two columns before the last one between
-      // the edges and put into columns C, -2 and -1 when they are needed.
-      const int jx = chi > 2 ? max(pj0, min(chi, C - 1) - 2) : 31;
+      // neighbours' words are put into columns C, -2 and -1 when they are needed.
       const bool rhalo = hasr && redge && it > first, lhalo = hasl && clo < 2 && it > first;
-      const unsigned events = (1u << jx) | (rhalo ? 1u << (C - 1) : 0u);
       const unsigned outs = (hasr ? 1u << (C - 1) : 0u) | (hasl ? 3u : 0u);
-      HT he[HR] = {};  // histories of the warp's columns below 2
-      auto fetch = [&]() {
-        if (rhalo) halo_fetch<1>(SH + 128, hin + hcta + 2 * hcol, hcol);
-        if (lhalo) halo_fetch<2>(SH, hin - hcta, hcol);
-        if (kB && clo < 2) {
-          he[0] = ldh(hp, clo, lsrc);
-          he[1] = ldh(hp, clo + 1, lsrc);
-        }
-      };
       auto put_left = [&]() {
-        if (!lhalo) return;
+        auto histories = [&]() {  // of the warp's columns below 2
+          if (!kB) return;
+          hq[0] = ldh(hp, clo, lsrc);
+          hq[1] = ldh(hp, clo + 1, lsrc);
+        };
+        if (!lhalo) {
+          histories();
+          return;
+        }
         Q4 h[2];
-        halo_get(SH, hin - hcta, hcol, tag - 1, poll, h);
+        halo_get(hin - hcta, hcol, tag - 1, poll, h, histories);
         sts4(F - 2 * FS, h[0]);
         sts4(F - FS, h[1]);
       };
       auto put_right = [&]() {
         Q4 r[1];
-        halo_get(SH + 128, hin + hcta + 2 * hcol, hcol, tag - 1, poll, r);
+        halo_get(hin + hcta + 2 * hcol, hcol, tag - 1, poll, r, [] {});
         sts4(F + FS * C, r[0]);
       };
       // Columns [j, je): four to an iteration, so that the window's registers
@@ -860,15 +856,11 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         const ulonglong2* cf = CF + 2 * j;
         u64* ed = ED + 2 * j;
         unsigned tp = TP + 8 * j, tk = TK + 4 * j, ho = (unsigned)((hoff + j * n1h) * kEs);
-        unsigned ev = events >> j, ot = outs >> j, ph = phys >> j, src = lsrc >> j;
+        unsigned ot = outs >> j, ph = phys >> j, src = lsrc >> j;
         int n = je - j;
         Q4 *sp0 = sptr[0] + j, *sp1 = sptr[1] + j;
         Q4 w0 = lds4(f - 2 * FS), w1 = lds4(f - FS), w2 = lds4(f), w3;
         auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
-          if (ev & (1u << k)) {
-            if (j + k == jx) fetch();
-            if (rhalo && j + k == C - 1) put_right();
-          }
           w3 = lds4(f + FS * (k + 1));
           const float4 z = up4(lds4(f + FS * k + 32));
           const float2 zm = up(fu[2 * FS * k]);
@@ -972,25 +964,31 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           tp += 32;
           tk += 16;
           ho += 4 * hstep;
-          ev >>= 4;
           ot >>= 4;
           ph >>= 4;
           src >>= 4;
         }
       };
-      for (int j = pj0, je = chi;;) {
-        if (j < 2) {
-          if (chi <= 2) fetch();  // else fetched at column jx
+#pragma unroll 1
+      for (int part = chi > 2 ? 0 : 2; part < 3; ++part) {  // the columns between, C - 1, 0 and 1
+        int j = pj0, je = rhalo ? C - 1 : chi;
+        if (part == 1) {
+          if (!rhalo) continue;
+          put_right();
+          if (kB && (C - 1 - pj0) % HR) {  // the quads read ahead go on where they are
+            const HT t = hq[0];
+            hq[0] = hq[1];
+            hq[1] = t;
+          }
+          j = C - 1;
+          je = C;
+        } else if (part == 2) {
+          if (clo > 1) break;
           put_left();
+          j = clo;
+          je = min(chi, 2);
         }
-        columns(j, je);
-        if (clo > 1 || je <= 2) break;
-        j = clo;  // the left edge's columns
-        je = 2;
-        if (kB) {
-          hq[0] = he[0];
-          hq[1] = he[1];
-        }
+        if (j < je) columns(j, je);
       }
       tm_wait_st();
       if (kA) {
@@ -1037,42 +1035,36 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         return add4(x, z);
       };
       // The warp's columns in order, column 0 last; the neighbours' words go into
-      // the tensor memory's columns C, C + 1 and -1.
-      const int jx = vj0 > 0 && vj0 < C - 1 ? max(vj0, min(chi, C - 2) - 2) : 31;
+      // the columns C, C + 1 and -1 of p.
       const bool rhalo = hasr && chi > C - 2, lhalo = hasl && ledge;
-      const unsigned events = (1u << jx) | (rhalo && clo <= C - 2 ? 1u << (C - 2) : 0u);
       const unsigned outs = (hasr ? 3u << (C - 2) : 0u) | (hasl ? 1u : 0u);
-      HT ex = {}, ez = {};  // histories of column 0
-      auto fetch = [&]() {
-        if (rhalo) halo_fetch<2>(SH + 128, hin + hcta + hcol, hcol);
-        if (lhalo) halo_fetch<1>(SH, hin - hcta, hcol);
-        if (kB && ledge) {
-          ex = ldh(hpx, 0, lphys);
-          ez = ldh(hpz, 0, lphys);
-        }
+      auto put_p = [&](int c, Q4 v) {
+        if (PS)
+          sts4(PP + 32 * c, v);
+        else
+          tm_st(TP + 8 * c, v, kZero4);
       };
       auto put_right = [&]() {
         Q4 r[2];
-        halo_get(SH + 128, hin + hcta + hcol, hcol, tag, poll, r);
-        if (PS) {
-          sts4(PP + 32 * C, r[0]);
-          sts4(PP + 32 * C + 32, r[1]);
-        } else {
-          tm_st(TP + 8 * C, r[0], kZero4);
-          tm_st(TP + 8 * C + 8, r[1], kZero4);
-          tm_wait_st();
-        }
+        halo_get(hin + hcta + hcol, hcol, tag, poll, r, [] {});
+        put_p(C, r[0]);
+        put_p(C + 1, r[1]);
+        if (!PS) tm_wait_st();
       };
       auto put_left = [&]() {
-        if (!lhalo) return;
-        Q4 h[1];
-        halo_get(SH, hin - hcta, hcol, tag, poll, h);
-        if (PS) {
-          sts4(PP - 32, h[0]);
-        } else {
-          tm_st(TP - 8, h[0], kZero4);
-          tm_wait_st();
+        auto histories = [&]() {  // of column 0
+          if (!kB) return;
+          hx[0] = ldh(hpx, 0, lphys);
+          hz[0] = ldh(hpz, 0, lphys);
+        };
+        if (!lhalo) {
+          histories();
+          return;
         }
+        Q4 h[1];
+        halo_get(hin - hcta, hcol, tag, poll, h, histories);
+        put_p(-1, h[0]);
+        if (!PS) tm_wait_st();
       };
       // Columns [j, je), as in the pressure half step.
       auto columns = [&](int j, int je) {
@@ -1081,14 +1073,10 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         const Q4* pp = PP + 32 * (j + 2);
         const u64* ed = ED + 2 * j;
         unsigned tp = TP + 8 * (j + 2), ho = (unsigned)((hoff + j * n1h) * kEs);
-        unsigned ev = events >> j, ot = outs >> j, ph = phys >> j, src = lphys >> j;
+        unsigned ot = outs >> j, ph = phys >> j, src = lphys >> j;
         int n = je - j;
         Q4 w0 = pload(j - 1), w1 = pload(j), w2 = pload(j + 1), w3;
         auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
-          if (ev & (1u << k)) {
-            if (j + k == jx) fetch();
-            if (rhalo && j + k == C - 2) put_right();
-          }
           const float4 p = up4(w1);
           float pm1 = __shfl_up_sync(kAll, p.w, 1);
           float n0 = __shfl_down_sync(kAll, p.x, 1), n1 = __shfl_down_sync(kAll, p.y, 1);
@@ -1178,29 +1166,33 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           tp += 32;
           pp += 4 * 32;
           ho += 4 * hstep;
-          ev >>= 4;
           ot >>= 4;
           ph >>= 4;
           src >>= 4;
         }
       };
-      for (int j = vj0, je = chi;;) {
-        if (j == 0) {
-          if (jx == 31) fetch();  // else fetched at column jx
-          put_left();
-        }
-        if (j == C - 1 && rhalo) {  // the last column is the warp's only one
-          fetch();
+#pragma unroll 1
+      for (int part = ledge && chi == 1 ? 2 : 0; part < 3; ++part) {  // ..., C - 2 and C - 1, 0
+        int j = vj0, je = rhalo ? C - 2 : chi;
+        if (part == 1) {
+          if (!rhalo) continue;
           put_right();
+          if (kB && vj0 < C - 2 && (C - 2 - vj0) % HR) {
+            const HT tx = hx[0], tz = hz[0];
+            hx[0] = hx[1];
+            hz[0] = hz[1];
+            hx[1] = tx;
+            hz[1] = tz;
+          }
+          j = max(vj0, C - 2);
+          je = chi;
+        } else if (part == 2) {
+          if (!ledge) break;
+          put_left();
+          j = 0;
+          je = 1;
         }
-        columns(j, je);
-        if (clo > 0 || je <= 1) break;
-        j = 0;  // column 0
-        je = 1;
-        if (kB) {
-          hx[0] = ex;
-          hz[0] = ez;
-        }
+        if (j < je) columns(j, je);
       }
       if (kA) {
         const unsigned mx = __reduce_max_sync(kAll, rows ? __float_as_uint(lmx) & 0x7fffffffu : 0u);
