@@ -304,6 +304,14 @@ void daw_hicks_locate(float z, float x, float hgrid, int32_t ofs, int32_t* out5)
  * failure path works.  No GPU fault is involved; the handle stays usable. */
 int daw_selftest_wait_timeout(daw_handle* h);
 
+/* Diagnostic (no counterpart in the reference), for the handle's later runs whose
+ * time loop stays on chip: their waits for another CTA's words give up after
+ * `polls` rounds (0 = the normal limit, some seconds; 1 makes about any run
+ * report DAW_ERR_TIMEOUT, without a GPU fault, and the handle stays usable),
+ * and their step tags go on from `step_tag` if that is ahead (0 = as they are;
+ * they start over from 1 past 0xe0000000). */
+int daw_selftest_onchip(daw_handle* h, int32_t polls, uint32_t step_tag);
+
 /* Library version string. */
 const char* daw_version(void);
 

@@ -281,6 +281,7 @@ struct daw_handle {
   int slot_datum = 0, slot_win = 0;
   bool slot_fp16 = false;
   unsigned res_tag = 1;  // next step tag of the on-chip time loops
+  int res_polls = kResPolls;
   // CTAs per SM of their kernels by (mode, FP16, density, p in shared memory, columns
   // per CTA, row blocks, shared memory)
   std::map<std::array<size_t, 7>, int> res_occ;
@@ -836,7 +837,8 @@ void check_device_error(daw_handle* h) {
     CK(cudaMemset(h->d_err, 0, sizeof(unsigned)));
     if (e & kErrTimeout)
       throw DawError{DAW_ERR_TIMEOUT,
-                     "a bounded device wait ran out (TMA tile copy did not complete)"};
+                     "a bounded device wait ran out (a TMA tile copy did not complete or, in an "
+                     "on-chip time loop, another CTA's words did not arrive)"};
     throw DawError{DAW_ERR_NAN, "non-finite value (NaN or Inf) in a stage-A wavefield history"};
   }
 }
@@ -1344,6 +1346,7 @@ void run_resident(daw_handle* h, Batch& b, int mode, const Window* w) {
   L.G = (g.n2e + L.C - 1) / L.C;
   L.RB = (g.n1e + 127) / 128;
   L.slo = mode == FM_STAGE_B_ES ? 1 : 0;
+  L.poll_limit = h->res_polls;
   L.n1h = hist_ld(h);
   L.hist_step0 = w && mode != FM_STAGE_A ? w->s0 : 0;
   L.err = h->d_err;
@@ -3001,6 +3004,13 @@ int daw_selftest_wait_timeout(daw_handle* h) {
     check_device_error(h);
   });
   return rc;
+}
+
+int daw_selftest_onchip(daw_handle* h, int32_t polls, uint32_t step_tag) {
+  if (!h || polls < 0) return DAW_ERR_ARG;
+  h->res_polls = polls ? polls : kResPolls;
+  if (step_tag) h->res_tag = std::max(h->res_tag, step_tag);  // no tag twice
+  return DAW_OK;
 }
 
 int daw_get_timing(const daw_handle* h, daw_timing* t) {

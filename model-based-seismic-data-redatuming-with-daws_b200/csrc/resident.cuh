@@ -10,6 +10,7 @@ constexpr int kResCols = 27;       // most grid columns per CTA (column masks re
 constexpr int kResRowBlocks = 15;  // most 128-row blocks per CTA
 constexpr int kResWarps = 16;      // most warps per CTA (128 registers a thread)
 constexpr int kResShots = 16;      // most shots (CTA groups) per launch
+constexpr int kResPolls = 1 << 22; // rounds after which a wait gives up (seconds)
 
 // A rectangle of the extended grid whose pressure every step is kept for the
 // Hicks gathers after the loop: rows [r0, r1), columns [c0, c1), step-major
@@ -51,6 +52,7 @@ struct ResidentLaunch {
   int CG, CW;                   // column groups and columns of a group (resident_launch)
   ulonglong2* halo;             // [phase][parity][cta][3][RB * 32][2]
   unsigned long long* slots;    // 72 words a CTA: stage A's maxima and their results
+  int poll_limit;               // kResPolls but in tests
   unsigned tag0;                // step tags of this launch: tag0 + step
   int load, save;               // state from / to global memory (else zero / dropped)
   int slo;                      // pressure source margin (1: final esource)

@@ -146,13 +146,14 @@ __device__ __forceinline__ u64 word_load(const u64* p) {
 // the limit is reached or another wait of the grid has run out.
 struct Poll {
   unsigned* err;
+  const int& limit;
   bool dead;
   __device__ __forceinline__ bool give_up(int n) {
-    if ((n & 255) != 255) return false;
+    if (n < limit && (n & 255) != 255) return false;
     unsigned e;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(e) : "l"(err) : "memory");
     // one decision for the warp: its lanes may see the flag at different times
-    dead = __any_sync(kAll, (e & kErrTimeout) != 0 || n > (1 << 22));
+    dead = __any_sync(kAll, (e & kErrTimeout) != 0 || n >= limit);
     if (dead && (threadIdx.x & 31) == 0) atomicOr(err, kErrTimeout);
     return dead;
   }
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   float* const SC = reinterpret_cast<float*>(sm + l.misc + 16 * 4);  // scales
   unsigned* const TB = reinterpret_cast<unsigned*>(sm + l.misc + 64 * 4);
   const unsigned top = lane == 0, bottom = lane == 31;
-  Poll poll{L.err, false};
+  Poll poll{L.err, L.poll_limit, false};
   const int4 ih = S.inj.pts > 0 ? S.inj.head[b] : make_int4(0, 0, 0, 0);
   const int ipts = ih.y > 0 ? C * ih.y : 0;
   const int im = L.inj_m;
