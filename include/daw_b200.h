@@ -76,8 +76,9 @@ enum daw_option {
                                 keeps whole histories. */,
   DAW_OPT_STEP_KERNEL = 9,   /* TMA kernel family (DAW_OPT_CHUNK = 0): 0 (default) =
                                 the time loop on chip where the grid fits the SMs'
-                                registers, shared and tensor memory, else from 5 Mi
-                                padded points on one kernel per time step, else (and
+                                shared and tensor memory (unless a batch of many shots
+                                of a small grid is faster in one launch), else from
+                                5 Mi padded points on one kernel per time step, else (and
                                 with DAW_OPT_PDL) separate pressure and velocity
                                 kernels, shots per launch and CTAs per SM chosen by the
                                 autotuner; 1 = one kernel
@@ -85,12 +86,14 @@ enum daw_option {
                                 stencil's halo, two alternating state sets), tile width
                                 and CTAs per SM autotuned; 2 = one or separate kernels,
                                 autotuned (the windows of a checkpointed shot then use
-                                the separate kernels) */
+                                the separate kernels); 3 = separate kernels */
   DAW_OPT_TILE_COLS = 10,    /* one-kernel-per-step tiles: 16 or 32 columns of 64
-                                rows; 0 (default) = chosen by the autotuner */
+                                rows; 0 (default) = chosen by the autotuner, 32 where
+                                the grid's size chose the family */
   DAW_OPT_CTAS_PER_SM = 11,  /* one-kernel-per-step CTAs per SM (1..3; a value above
                                 what fits is lowered to the occupancy); 0 (default) =
-                                chosen by the autotuner */
+                                chosen by the autotuner, the occupancy where the grid's
+                                size chose the family */
   DAW_OPT_PDL = 12           /* TMA kernels: 1 = programmatic dependent launch (a time
                                 step's kernel starts launching while the previous one
                                 drains); 0 (default) = plain stream order */

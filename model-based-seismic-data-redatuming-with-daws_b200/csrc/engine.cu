@@ -725,7 +725,9 @@ int chunk_of(const daw_handle* h) { return h->opt.chunk; }
 // kernels' then and where the family is autotuned (DAW_OPT_STEP_KERNEL = 2).
 bool tma_path(const daw_handle* h) { return h->opt.fused && h->opt.chunk == 0; }
 bool split_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && h->opt.step != 1 && !b.step; }
-bool step_maps(const daw_handle* h, const Batch& b) { return tma_path(h) && (h->opt.step != 0 || b.step); }
+bool step_maps(const daw_handle* h, const Batch& b) {
+  return tma_path(h) && (h->opt.step == 1 || h->opt.step == 2 || b.step);
+}
 // Family of the windows of a checkpointed shot (not tuned): the step kernels
 // when pinned or chosen by the grid's size.
 bool windowed_step(const daw_handle* h, const Batch& b) { return tma_path(h) && (h->opt.step == 1 || b.step); }
@@ -951,7 +953,7 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
     timed = true;
     if (cd.us_per_step < best.us_per_step) best = cd;
   };
-  if (h->opt.step != 1 && !b.step) {
+  if (h->opt.step != 1) {
     // shots per launch (default shapes), then the CTAs per SM for the best
     std::vector<int> ks;
     for (int k : {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64})
@@ -965,7 +967,7 @@ daw_handle::Tuned tune_run(daw_handle* h, Batch& b, int mode, FusedLaunch L, int
         for (int vc = 1; vc <= occ_v; ++vc)
           if (!(timed && pc == occ_p && vc == occ_v)) consider({0, 32, pc, vc, kbest, 0.f});
   }
-  if ((h->opt.step != 0 || b.step) && !h->md.rbw1)  // the step family has no density variant
+  if ((h->opt.step == 1 || h->opt.step == 2) && !h->md.rbw1)  // the step family has no density variant
     for (int tc : {16, 32}) {
       if (h->opt.tile_cols && h->opt.tile_cols != tc) continue;
       // a pinned CTA count above what fits is clamped to the occupancy
@@ -2637,8 +2639,8 @@ int daw_set_option(daw_handle* h, int32_t key, double value) {
         h->opt.checkpoint = v;
         break;
       case DAW_OPT_STEP_KERNEL:
-        if (v < 0 || v > 2)
-          throw DawError{DAW_ERR_ARG, "step kernel: 0 split, 1 one per step, 2 autotuned"};
+        if (v < 0 || v > 3)
+          throw DawError{DAW_ERR_ARG, "step kernel: 0 by the grid, 1 one per step, 2 autotuned, 3 split"};
         h->opt.step = v;
         break;
       case DAW_OPT_PDL: h->opt.pdl = v ? 1 : 0; break;
