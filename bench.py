@@ -24,7 +24,7 @@ model on the GPU before timing.  Density is 1 as in the reference
 stage-in is untimed).  `e2e`: the same shots through daw_shots with host
 buffers, host-device copies included.  Denominators on the first timed
 batch's shots: `plain_fp32` (kernel per reference loop, FP32 histories and
-scalars) and `fused_fp32` (the same one-kernel-per-step kernels with FP32
+scalars) and `fused_fp32` (the same kernels as the timed path, with FP32
 histories and FP32 scalars).  `accuracy`: the mixed path against the FP64
 oracle on the whole 151x461 single-shot configuration, and against the
 FP32-history kernels on the timed batch.  The reference arm (--impl
@@ -53,8 +53,8 @@ sys.path.insert(0, ROOT)
 import __graft_entry__ as entry  # noqa: E402
 
 PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
-# DRAM bytes per shot time step of the pressure + velocity kernels, measured
-# by ncu on the same grid
+# DRAM bytes per shot time step of the separate pressure + velocity kernels,
+# measured by ncu on the 751x2301 grid
 TRAFFIC = os.path.join(ROOT, "profiles", "k_tma_751x2301_traffic.json")
 METRIC = "shots/hour redatumed at <=1e-3 rel err vs FP64: batched mixed vs plain FP32"
 
@@ -345,19 +345,27 @@ def op_steps_per_application(nt, window):
 
 
 def roofline(tim, w, fp16=True, rho=False):
-    """The step kernels of the G G^T stages (stage A and stage B, one launch
-    per time step): algorithmic bytes per shot step = 36 B per extended point
-    (px, pz, vx, vz read and written, kappa read) + 3 history fields per
-    interior point (written in stage A, read in stage B: 2 B each in FP16),
-    over the device time of those time loops.  With a density, the two
-    buoyancy coefficient fields add 8 B per extended point, and the buoyancy
-    weight of stage B's velocity sources 4 B per interior point of a stage-B
-    step."""
+    """The time loops of the G G^T stages (stage A and stage B) over their
+    device time.
+
+    From global memory (one or two kernels per time step): algorithmic bytes
+    per shot step = 36 B per extended point (px, pz, vx, vz read and written,
+    kappa read) + 3 history fields per interior point (written in stage A,
+    read in stage B: 2 B each in FP16).  With a density, the two buoyancy
+    coefficient fields add 8 B per extended point, and the buoyancy weight of
+    stage B's velocity sources 4 B per interior point of a stage-B step.
+
+    On chip the fields stay in shared and tensor memory and the neighbours'
+    words in L2: what a shot step moves through HBM is its histories (and the
+    density's coefficients), and HBM is not what bounds it."""
     peaks = json.load(open(PEAKS)) if os.path.exists(PEAKS) else {}
     peak = peaks.get("hbm_gbs", 6650.0)
+    family = tim.get("kernel_family", [0] * 4)[1]  # stage A's; stage B has the same
     ne = (w.n1 + 2 * w.npml) * (w.n2 + 2 * w.npml)
     ni = w.n1 * w.n2
-    per_shot_step = 36.0 * ne + 3 * (2 if fp16 else 4) * ni + (8.0 * ne if rho else 0.0)
+    per_shot_step = 3 * (2 if fp16 else 4) * ni + (8.0 * ne if rho else 0.0)
+    if family != 2:
+        per_shot_step += 36.0 * ne
     shot_steps = tim["shot_steps_a"] + tim["shot_steps_b"]
     if rho:  # averaged over the stage-A and stage-B shot steps
         per_shot_step += 4.0 * ni * tim["shot_steps_b"] / max(shot_steps, 1)
@@ -367,23 +375,27 @@ def roofline(tim, w, fp16=True, rho=False):
     avg_ms = ms / max(launches, 1)
     bytes_per_launch = per_shot_step * shot_steps / max(launches, 1)
     traffic, note = None, None
-    if rho:
-        note = "the committed ncu traffic capture ran rho = 1; none for this density"
+    if rho or family != 0 or (w.n1, w.n2) != (751, 2301):
+        note = ("the committed ncu traffic capture is of the separate kernels on 751x2301 with "
+                "rho = 1; none for these kernels")
     elif os.path.exists(TRAFFIC):
         t = json.load(open(TRAFFIC))
         traffic = t["bytes_per_shot_step"] * shot_steps / max(launches, 1)
         note = t["note"]
-    return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    unit = {0: "one time step of every shot of the launch (a pressure and a velocity kernel)",
+            1: "one launch of the step kernel (one time step of every shot of the batch)",
+            2: "one time step of the shots that share an on-chip launch"}[family]
+    return {"bound": "instruction issue and latency on chip" if family == 2 else "hbm",
+            "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "traffic": traffic, "traffic_note": note,
             "peak_source": "measured" if peaks else "fallback",
-            "unit_of_work": "one launch of the step kernel (one time step of every shot of the "
-                            "batch) in the G G^T stages",
+            "unit_of_work": unit + " in the G G^T stages",
             "bytes_per_launch": bytes_per_launch, "avg_launch_ms": avg_ms,
             "bytes_per_shot_step": per_shot_step}
 
 
 def reference_runs(pkg, local, shots, base_out):
-    """The plain FP32 port and the FP32-history step kernels on `shots`, one
+    """The plain FP32 port and the same kernels with FP32 histories on `shots`, one
     staged batch at a time; shots/hour of each and the mixed path's error
     against the FP32-history outputs."""
     res = {}
@@ -463,7 +475,7 @@ def run_ours(args):
     mine = list(range(ista - 1, iend))
     cap = args.batch if args.config == 2 else 8
     h = pkg.Handle(local, preset="mixed", checkpoint=args.checkpoint,
-                   step={"split": 0, "step": 1, "auto": 2}[args.kernel], tile_cols=args.tile_cols,
+                   step={"default": 0, "step": 1, "auto": 2, "split": 3}[args.kernel], tile_cols=args.tile_cols,
                    ctas_per_sm=args.ctas_per_sm, pdl=1 if args.pdl else 0)
     if args.config in (2, 5):
         per_step = args.batch
@@ -637,14 +649,16 @@ def run_ours(args):
             "config": bench_config(w, args, world),
             "run": {"shots_per_step": [int(x) for x in step_shots],
                     "shots_timed": int(shots_done),
-                    "kernel": {"auto": "TMA time-step kernels, family and launch shape "
-                                       "autotuned per mode",
+                    "kernel": {"default": "by the grid: time loops on chip, one or two kernels "
+                                          "per time step",
+                               "auto": "one or two TMA kernels per time step, family and "
+                                       "launch shape autotuned per mode",
                                "split": "TMA pressure and velocity kernels, shots per launch "
                                         "and CTAs per SM autotuned per mode",
                                "step": "one TMA kernel per time step (p recomputed on the "
                                        "v halo)"}[args.kernel]
                               + (", programmatic dependent launch" if args.pdl else ""),
-                    "autotuned": tc},
+                    "kernels": tc},
             "clocks": clk.summary(),
             "e2e": e2e,
             "gpu_launches": int(tim["kernel_launches"]),
@@ -711,9 +725,9 @@ def main():
     ap.add_argument("--nt", type=int, default=7500)
     ap.add_argument("--maxiter", type=int, default=None)
     ap.add_argument("--no-e2e", action="store_true")
-    # A/B: the one-kernel-per-step path (default) or the split p / v kernels
-    # the TMA kernel family: autotuned (default), split p / v kernels, or one per step
-    ap.add_argument("--kernel", default="split", choices=["split", "step", "auto"])
+    # the kernel family: by the grid, or pinned: split p / v kernels, one kernel per step, the
+    # faster of these two
+    ap.add_argument("--kernel", default="default", choices=["default", "split", "step", "auto"])
     ap.add_argument("--pdl", action="store_true",
                     help="programmatic dependent launch between steps (default: stream order)")
     # pin the step kernel's tile width / CTAs per SM (0 = autotuned)
