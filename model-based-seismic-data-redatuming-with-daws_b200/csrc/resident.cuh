@@ -1,5 +1,6 @@
 // Time loops on chip (stencil_resident.cu): a shot's whole wavefield stays in
-// the shared and tensor memory of a group of CTAs for all steps of a launch.  This header is what the engine needs to plan and launch them.
+// the shared and tensor memory of a group of CTAs for all steps of a launch.
+// This header is what the engine needs to plan and launch them.
 #pragma once
 
 #include "fused.cuh"

@@ -554,18 +554,14 @@ __global__ void __launch_bounds__(256)
       const int c = q / nv, r = (q - c * nv) * V;
       const size_t o = (size_t)it * 3 * field_stride + (size_t)inner_ld * (c0 + c) + r;
       float v[V];
-      if (FP16) {
-        if constexpr (V == 8) {
-          const uint4 x = __ldcs(reinterpret_cast<const uint4*>(static_cast<const __half*>(hist) + o));
-          const unsigned w[4] = {x.x, x.y, x.z, x.w};
+      if constexpr (FP16) {
+        const uint4 x = __ldcs(reinterpret_cast<const uint4*>(static_cast<const __half*>(hist) + o));
+        const unsigned w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
-            v[2 * k] = f.x;
-            v[2 * k + 1] = f.y;
-          }
-        } else {
-          v[0] = __half2float(static_cast<const __half*>(hist)[o]);
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+          v[2 * k] = f.x;
+          v[2 * k + 1] = f.y;
         }
       } else {
         if constexpr (V == 4) {
@@ -671,14 +667,14 @@ void history_cost(const void* hist, int fp16, const unsigned* amax, int nt, int 
                   cudaStream_t st) {
   const int blocks = 148 * 8;
   // whole 16-byte loads where columns start at 16-byte boundaries: always in the
-  // fused kernels' layout, by chance in the plain kernels'
-  const int v = fp16 ? 8 : 4;
-  const bool wide = inner_ld % v == 0 && field_stride % v == 0;
+  // fused kernels' layout (columns of a multiple of 8 values), which FP16 histories
+  // have, by chance in the plain kernels'
+  const bool wide = inner_ld % 4 == 0 && field_stride % 4 == 0;
   auto run = [&](auto k) {
     k<<<blocks, 256, 0, st>>>(hist, amax, nt, n1, n2, inner_ld, inner_off, field_stride, out);
   };
   if (fp16)
-    wide ? run(k_hist_cost<true, 8>) : run(k_hist_cost<true, 1>);
+    run(k_hist_cost<true, 8>);
   else
     wide ? run(k_hist_cost<false, 4>) : run(k_hist_cost<false, 1>);
 }
