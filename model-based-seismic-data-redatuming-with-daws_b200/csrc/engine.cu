@@ -1251,11 +1251,17 @@ ResidentShape resident_shape(daw_handle* h, const Batch& b, int mode) {
                          resident_smem(b.res_cols, s.RB, ps, s.pts, s.m, s.nsta, s.quads));
   };
   s.occ = occupancy(false);
-  // where it has room: stage B 151 x 461 3.04 to 2.68 us a step, 647 x 1533 6.84 to
-  // 6.59, 301 x 703 the same; both stages with FP32 histories 3.40 to 3.21 and 3.24
-  // to 2.80.  The forward run gains nothing and stage A with FP16 histories loses
-  // (registers spill: 3.7 to 4.2): they have no such variant.
-  s.ps = occupancy(true) >= s.occ;
+  // Where it has room, and where it lets more warps work or loads the SMs' quadrants
+  // evenly (one to three and five to seven row blocks).  us per step of stage B, and of
+  // stage A with FP32 histories, without and with it:
+  //   30 x 1500   4.45 3.04  4.81 2.65     301 x 703   3.29 3.42  3.70 3.66
+  //   120 x 1500  4.49 3.75  4.44 3.46     400 x 900   3.92 4.17  4.27 4.43 (not taken)
+  //   151 x 461   2.93 2.69  3.07 2.80     500 x 1000  5.39 4.85  5.62 4.87
+  //   250 x 1200  4.10 3.93  4.68 3.83     647 x 1533  6.50 6.13  8.18 7.42
+  //   1000 x 200  5.84 6.18  5.86 5.92 (not taken)
+  // The forward run gains nothing and stage A with FP16 histories loses (registers
+  // spill): they have no such variant.
+  s.ps = s.RB < 8 && s.RB % 4 != 0 && occupancy(true) >= s.occ;
   s.room = s.occ * h->sms / s.G;
   return s;
 }

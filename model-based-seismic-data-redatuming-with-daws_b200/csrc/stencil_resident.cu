@@ -53,9 +53,9 @@
 // neighbours' words waited for inside the edge column after what does not need
 // them (stage A 3.9 us against 3.7 at 151 x 461: registers spill).
 // Measured per shot step against the split kernels (B200, FP16 histories):
-// 751 x 2301 (17 columns a CTA) forward 7.0 us against 20.1, stage A 10.7
-// against 20.7-23.0, stage B 8.7 against 19.7-24.7; 151 x 461 (4 columns)
-// 2.4-3.7 us against 12-15.
+// 751 x 2301 (17 columns a CTA) forward 7.1 us against 20.1, stage A 10.8
+// against 20.7-23.0, stage B 8.4 against 19.7-24.7; 151 x 461 (4 columns)
+// 2.1-3.8 us against 12-15.
 #include <algorithm>
 
 #include "resident.cuh"
@@ -159,18 +159,8 @@ struct Poll {
   }
 };
 
-// N halo columns at p, p + stride, ...: polled until all words carry the tag, between
-// the parts of a warp's columns (in the column code itself the wait is there four times
-// over: instruction cache).  us per step of forward / stage A / stage B, 751 x 2301 6.93
-// / 10.9 / 8.37, 301 x 703 2.59 / 4.12 / 3.42, 151 x 461 2.20 / 3.7 / 2.57.  Tried:
-// - in the column code 7.20 / 10.9 / 9.19, 2.57 / 4.2 / 3.86, 2.12 / 3.8 / 2.78;
-// - there, copied to shared memory a few columns ahead by cp.async, which is a weak access
-//   and races with the neighbour's store in the memory model: 7.13 / 10.7 / 8.78, 2.56 /
-//   4.2 / 3.49, 2.27 / 3.7 / 2.69;
-// - loaded a few columns ahead and put into shared memory by the lane, at once: 7.80 /
-//   11.6 / 9.62, 2.85 / 4.3 / 4.08, 2.40 / 3.9 / 3.18; at the end of the column: stage B
-//   11.5, 4.44, 3.51 (registers spill);
-// - copied by the extra warp: forward and stage B 10.6 / 12.1, 4.75 / 6.6, 3.56 / 5.0.
+// N halo columns at p, p + stride, ...: polled until all words carry the tag; other
+// loads may go out with the first round (`meanwhile`).
 template <int N, typename F>
 __device__ __forceinline__ void halo_get(const ulonglong2* p, size_t stride, unsigned tag, Poll& w,
                                          Q4 (&v)[N], F&& meanwhile) {
@@ -428,7 +418,7 @@ __host__ __device__ inline Lay layout(int C, int RB, int pts, int m, int nsta, i
 //   leave some idle.
 // - In shared memory too (PS, where it has room: 512 bytes per column and row
 //   block): tensor memory is private to a warp and the warps fill the quadrants
-//   in turn.  Stage B 151 x 461 3.04 to 2.68 us a step.
+//   in turn.
 __host__ __device__ inline int group_warps(int RB, bool ps) { return ps ? RB : (RB + 3) / 4 * 4; }
 __host__ __device__ inline int cta_warps(int RB, int CG, bool ps) {
   return !ps && RB % 4 ? CG * group_warps(RB, ps) : CG * group_warps(RB, ps) + 1;
@@ -474,6 +464,20 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
   constexpr bool kA = MODE == FM_STAGE_A, kB = MODE == FM_STAGE_B, kF = MODE == FM_FWD;
   constexpr int FS = 64;  // quads between a lane's columns
   constexpr int HR = 2;   // history columns read ahead
+  // The wait for the right neighbour's words stands between two parts of a warp's columns,
+  // or in the column code, four times over.  us per step with parts and without:
+  //              751 x 2301   600 x 600    301 x 703    151 x 461
+  //   forward     6.93  7.12   3.43  3.15   2.59  2.52   2.20  2.11
+  //   A, FP16    10.9  10.8    4.99  4.71   4.12  3.96   3.7   3.8
+  //   A, FP32    10.5  10.9    3.71  3.97   3.66  4.05   2.81  2.98
+  //   B           8.41  9.19   4.15  4.10   3.45  3.86   2.63  2.78
+  // Tried in place of the wait, stage B at 751 x 2301:
+  // - the words copied to shared memory a few columns ahead by cp.async, which is a weak
+  //   access and races with the neighbour's store in the memory model: 8.78;
+  // - loaded a few columns ahead and put into shared memory by the lane, at once: 9.62; at
+  //   the end of the column: 11.5 (registers spill);
+  // - copied by the extra warp: 12.1.
+  constexpr bool kParts = kB || (kA && !FP16);
   using HQ = HQuad<FP16>;
   using HT = typename HQ::T;
   extern __shared__ __align__(16) unsigned char sm[];
@@ -847,6 +851,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         halo_get(hin + hcta + 2 * hcol, hcol, tag - 1, poll, r, [] {});
         sts4(F + FS * C, r[0]);
       };
+      const unsigned wait = !kParts && rhalo ? 1u << (C - 1) : 0u;
       // Columns [j, je): four to an iteration, so that the window's registers
       // rotate without copies.  Arrays at column j, masks shifted by j.
       auto columns = [&](int j, int je) {
@@ -857,11 +862,12 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         const ulonglong2* cf = CF + 2 * j;
         u64* ed = ED + 2 * j;
         unsigned tp = TP + 8 * j, tk = TK + 4 * j, ho = (unsigned)((hoff + j * n1h) * kEs);
-        unsigned ot = outs >> j, ph = phys >> j, src = lsrc >> j;
+        unsigned ev = wait >> j, ot = outs >> j, ph = phys >> j, src = lsrc >> j;
         int n = je - j;
         Q4 *sp0 = sptr[0] + j, *sp1 = sptr[1] + j;
         Q4 w0 = lds4(f - 2 * FS), w1 = lds4(f - FS), w2 = lds4(f), w3;
         auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
+          if (!kParts && (ev & (1u << k))) put_right();
           w3 = lds4(f + FS * (k + 1));
           const float4 z = up4(lds4(f + FS * k + 32));
           const float2 zm = up(fu[2 * FS * k]);
@@ -965,16 +971,26 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           tp += 32;
           tk += 16;
           ho += 4 * hstep;
+          if (!kParts) ev >>= 4;
           ot >>= 4;
           ph >>= 4;
           src >>= 4;
         }
       };
+      if (!kParts) {
+        for (int j = pj0, je = chi;;) {
+          if (j < 2) put_left();
+          columns(j, je);
+          if (clo > 1 || je <= 2) break;
+          j = clo;  // the left edge's columns
+          je = 2;
+        }
+      } else {
 #pragma unroll 1
       for (int part = chi > 2 ? 0 : 2; part < 3; ++part) {  // the columns between, C - 1, 0 and 1
-        int j = pj0, je = rhalo ? C - 1 : chi;
+        int j = pj0, je = kParts && rhalo ? C - 1 : chi;
         if (part == 1) {
-          if (!rhalo) continue;
+          if (!kParts || !rhalo) continue;
           put_right();
           if (kB && (C - 1 - pj0) % HR) {  // the quads read ahead go on where they are
             const HT t = hq[0];
@@ -990,6 +1006,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           je = min(chi, 2);
         }
         if (j < je) columns(j, je);
+      }
       }
       tm_wait_st();
       if (kA) {
@@ -1052,6 +1069,7 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         put_p(C + 1, r[1]);
         if (!PS) tm_wait_st();
       };
+      const unsigned wait = !kParts && rhalo && clo <= C - 2 ? 1u << (C - 2) : 0u;
       auto put_left = [&]() {
         auto histories = [&]() {  // of column 0
           if (!kB) return;
@@ -1074,10 +1092,11 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
         const Q4* pp = PP + 32 * (j + 2);
         const u64* ed = ED + 2 * j;
         unsigned tp = TP + 8 * (j + 2), ho = (unsigned)((hoff + j * n1h) * kEs);
-        unsigned ot = outs >> j, ph = phys >> j, src = lphys >> j;
+        unsigned ev = wait >> j, ot = outs >> j, ph = phys >> j, src = lphys >> j;
         int n = je - j;
         Q4 w0 = pload(j - 1), w1 = pload(j), w2 = pload(j + 1), w3;
         auto column = [&](const int k, const Q4& w0, const Q4& w1, const Q4& w2, Q4& w3) {
+          if (!kParts && (ev & (1u << k))) put_right();
           const float4 p = up4(w1);
           float pm1 = __shfl_up_sync(kAll, p.w, 1);
           float n0 = __shfl_down_sync(kAll, p.x, 1), n1 = __shfl_down_sync(kAll, p.y, 1);
@@ -1167,16 +1186,27 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           tp += 32;
           pp += 4 * 32;
           ho += 4 * hstep;
+          if (!kParts) ev >>= 4;
           ot >>= 4;
           ph >>= 4;
           src >>= 4;
         }
       };
+      if (!kParts) {
+        for (int j = vj0, je = chi;;) {
+          if (j == 0) put_left();
+          if (j == C - 1 && rhalo) put_right();  // the warp's only column: p of column C before it starts
+          columns(j, je);
+          if (clo > 0 || je <= 1) break;
+          j = 0;  // column 0
+          je = 1;
+        }
+      } else {
 #pragma unroll 1
       for (int part = ledge && chi == 1 ? 2 : 0; part < 3; ++part) {  // ..., C - 2 and C - 1, 0
-        int j = vj0, je = rhalo ? C - 2 : chi;
+        int j = vj0, je = kParts && rhalo ? C - 2 : chi;
         if (part == 1) {
-          if (!rhalo) continue;
+          if (!kParts || !rhalo) continue;
           put_right();
           if (kB && vj0 < C - 2 && (C - 2 - vj0) % HR) {
             const HT tx = hx[0], tz = hz[0];
@@ -1193,7 +1223,10 @@ __global__ void __launch_bounds__(32 * kResWarps, 1)
           j = 0;
           je = 1;
         }
+        // the last column is the warp's only one: p of column C before it starts
+        if (!kParts && rhalo && j == C - 1) put_right();
         if (j < je) columns(j, je);
+      }
       }
       if (kA) {
         const unsigned mx = __reduce_max_sync(kAll, rows ? __float_as_uint(lmx) & 0x7fffffffu : 0u);
